@@ -392,13 +392,26 @@ CGArgs step_cg_args(yk_ctx* ctx)
     return a;
 }
 
+// The one lattice of every system of the step (Nt 0: they differ).
+OneLattice step_lattice(const yk_ctx* ctx)
+{
+    OneLattice q = {};
+    for (const Chain& C : ctx->ch) {
+        if (C.n_rhs_step == 0) continue;
+        if (q.Nt && (q.Nt != C.Nt || q.Nx != C.Nx)) return {};
+        q.Nt = C.Nt;
+        q.Nx = C.Nx;
+    }
+    return q;
+}
+
 int enqueue_step(yk_ctx* ctx)
 {
     cudaEvent_t e = nullptr;
     NoiseTables nt = {ctx->d_rows, ctx->nrows, ctx->d_cols, ctx->ncols, ctx->d_white, ctx->nwhite};
     int free_sm = 0;
     if (ctx->noise_overlap && !ctx->profiling && !ctx->cg_cluster && ctx->nsys > 0 && ctx->nrows > 0)
-        free_sm = ctx->n_sm - cg_predict_grid(step_cg_args(ctx), ctx->precision == YK_MIXED);
+        free_sm = ctx->n_sm - cg_predict_grid(step_cg_args(ctx), ctx->precision == YK_MIXED, step_lattice(ctx));
     const bool overlap = free_sm >= 8 && ctx->overlap_choice != 0;
     if (overlap) {
         YK_CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
@@ -426,7 +439,8 @@ int enqueue_step(yk_ctx* ctx)
             // batched: block ranges balanced by the previous step's iterations
             const bool bal = ctx->nsys > 1 && ctx->cg_balance && !ctx->cg_eo;
             if (bal) a.balance = ctx->d_balance;
-            YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, &ctx->cg_grid, &ctx->cg_kernel));
+            YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, &ctx->cg_grid, &ctx->cg_kernel,
+                            step_lattice(ctx)));
             if (bal) YK_CK(launch_cg_balance(a, ctx->cg_grid, ctx->d_balance, ctx->stream));
             prof_end(ctx, 1, e, bal ? 3 : 2);
         }
@@ -568,7 +582,7 @@ int ws_solve(yk_ctx* ctx, int c, int count, int mtype, double tol, int tol_mode,
     a.tol = tol;
     a.tol_mode = tol_mode;
     a.max_iter = max_iter;
-    YK_CK(launch_cg(a, 2, precision == YK_MIXED, ctx->stream, nullptr));
+    YK_CK(launch_cg(a, 2, precision == YK_MIXED, ctx->stream, nullptr, nullptr, {C.Nt, C.Nx, C.pions ? 1 : 0}));
     std::vector<CGState> st(count);
     YK_CK(cudaMemcpyAsync(st.data(), w.d_state, sizeof(CGState) * count, cudaMemcpyDeviceToHost, ctx->stream));
     int rc = status_of_err(ctx);
@@ -623,7 +637,7 @@ int chain_solve(yk_ctx* ctx, int c, int kind, yk_solve_stats* stats, bool want_x
         YK_CK(launch_eta(ctx->d_sys, ctx->d_sys_tiles + C.cg_tile0, C.cg_tile1 - C.cg_tile0, kind, ctx->stream));
         YK_CK(launch_cg_cluster(a, ctx->cluster_sites, ctx->stream));
     } else {
-        YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, nullptr));
+        YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, nullptr, nullptr, {C.Nt, C.Nx, 0}));
     }
     std::vector<CGState> st(C.n_rhs_step);
     YK_CK(cudaMemcpyAsync(st.data(), ctx->d_state + C.sys0, sizeof(CGState) * C.n_rhs_step,
@@ -660,7 +674,7 @@ int tune_overlap(yk_ctx* ctx)
 {
     yk_tune_result& T = ctx->tune;
     if (!ctx->noise_overlap || ctx->cg_cluster || ctx->nsys == 0 || ctx->nrows == 0 || ctx->pions) return YK_OK;
-    if (ctx->n_sm - cg_predict_grid(step_cg_args(ctx), ctx->precision == YK_MIXED) < 8) return YK_OK;
+    if (ctx->n_sm - cg_predict_grid(step_cg_args(ctx), ctx->precision == YK_MIXED, step_lattice(ctx)) < 8) return YK_OK;
     const int nch = (int)ctx->ch.size();
     size_t nphi = 0;
     for (const Chain& C : ctx->ch) nphi += (size_t)C.V;
@@ -761,9 +775,9 @@ int run_autotune(yk_ctx* ctx)
             if (c < 8 || c > maxg) continue;
             if ((ctx->n_sys_tiles + c - 1) / c > kMaxTilesPerBlock) continue;
             a.grid_cap = c;
-            cudaError_t e = launch_cg(a, 1, mixed, ctx->stream, nullptr);
+            cudaError_t e = launch_cg(a, 1, mixed, ctx->stream, nullptr, nullptr, step_lattice(ctx));
             if (e == cudaSuccess) e = cudaEventRecord(e0, ctx->stream);
-            for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep) e = launch_cg(a, 1, mixed, ctx->stream, nullptr);
+            for (int rep = 0; rep < 2 && e == cudaSuccess; ++rep) e = launch_cg(a, 1, mixed, ctx->stream, nullptr, nullptr, step_lattice(ctx));
             if (e == cudaSuccess) e = cudaEventRecord(e1, ctx->stream);
             if (e == cudaSuccess) e = cudaEventSynchronize(e1);
             float ms = 0.f;
@@ -1043,6 +1057,7 @@ int yk_ctx_create(const yk_params* params, int n_chains, yk_ctx** out)
     cg_max_grid(2, false);
     cg_max_grid(2, true);
     if (mixed) cg_halo_init();
+    cg_small_init();
     noise_init_attributes();
     {
         // opt-in while its FP64 reliable updates run on 16 SMs only

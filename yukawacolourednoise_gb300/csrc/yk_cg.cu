@@ -4469,7 +4469,7 @@ static bool eo_single_variant(const CGArgs& a, int* px, int* grid, int* tpb, siz
 
 // The grid launch_cg would use for `a` (the even-odd kernels' when the caller
 // gave the compact views, as launch_cg_t picks them).
-int cg_predict_grid(const CGArgs& a, bool mixed)
+int cg_predict_grid(const CGArgs& a, bool mixed, const OneLattice& lat)
 {
     if (mixed && a.sys_eo && a.eo_tiles && a.mtype == YK_DAGGER && a.balance == nullptr &&
         a.sys_count <= kEobMaxSys) {
@@ -4481,6 +4481,7 @@ int cg_predict_grid(const CGArgs& a, bool mixed)
         if (a.eo_patches && !(pe && pe[0] == '0') && eop_max_grid() > 0) return std::min(capped(eop_max_grid(), a.grid_cap), std::max(nt, 1));
         return std::min(capped(eob_max_grid(), a.grid_cap), std::max((nt + 1) / 2, 1));
     }
+    if (const int g = cg_small_grid(a, 1, mixed, lat)) return g;
     int tpb = 1;
     return cg_grid_for(a.tile_end - a.tile_begin,
                        capped(mixed ? max_grid_t<1, true>() : max_grid_t<1, false>(), a.grid_cap), &tpb);
@@ -4728,8 +4729,14 @@ cudaError_t launch_cg_balance(const CGArgs& a, int grid, int* out, cudaStream_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_cg(const CGArgs& a, int K, bool mixed, cudaStream_t stream, int* grid_out, int* kernel_out)
+cudaError_t launch_cg(const CGArgs& a, int K, bool mixed, cudaStream_t stream, int* grid_out, int* kernel_out,
+                      const OneLattice& lat)
 {
+    if (const int g = cg_small_grid(a, K, mixed, lat)) {
+        if (grid_out) *grid_out = g;
+        if (kernel_out) *kernel_out = 6;
+        return launch_cg_small(a, K, mixed, lat, stream);
+    }
     if (K == 1)
         return mixed ? launch_cg_t<1, true>(a, stream, grid_out, kernel_out)
                      : launch_cg_t<1, false>(a, stream, grid_out, kernel_out);

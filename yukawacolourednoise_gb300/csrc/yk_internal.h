@@ -150,6 +150,12 @@ struct CGArgs {
     int eo;
 };
 
+// The one lattice of all systems of a solve, for cg_small_kernel (Nt 0: they differ).
+struct OneLattice {
+    int Nt, Nx;
+    int pions;   // whether they carry pions
+};
+
 // Per-chain device record of the Langevin step.
 struct ChainDev {
     int Nt, Nx, V;

@@ -17,8 +17,17 @@ cudaError_t launch_dirac(const void* in, void* out, const double* sigma, int Nt,
 
 // Batched CG (yk_cg.cu).  Also launches its one-block preparation kernel.
 // grid_out: blocks launched; kernel_out: 0 cg_kernel, 1 cg_halo_kernel, 3 cg_eo_kernel
-// (the even-odd solve: a.sys_eo given, chi = (D^dag)^-1 b left in t64) (either may be null)
-cudaError_t launch_cg(const CGArgs& a, int K, bool mixed, cudaStream_t stream, int* grid_out, int* kernel_out = nullptr);
+// (the even-odd solve: a.sys_eo given, chi = (D^dag)^-1 b left in t64), 6 cg_small_kernel
+// (either may be null)
+cudaError_t launch_cg(const CGArgs& a, int K, bool mixed, cudaStream_t stream, int* grid_out, int* kernel_out = nullptr,
+                      const OneLattice& lat = {});
+// The CG of small lattices inside one cluster per system (yk_cg_small.cu),
+// which launch_cg takes for FP64 and for complex solves when every vector fits:
+// its grid for `a` (0: not taken), its launch, and the kernels' attributes
+// (call before any stream capture).
+int cg_small_grid(const CGArgs& a, int K, bool mixed, const OneLattice& lat);
+cudaError_t launch_cg_small(const CGArgs& a, int K, bool mixed, const OneLattice& lat, cudaStream_t stream);
+void cg_small_init();
 // Work-balanced block ranges (CGArgs::balance) for the next solve of the
 // systems of `a`, from their iteration counts in the solve just finished;
 // grid: the grid of that solve's launch.  No-op for a single system.
@@ -57,7 +66,7 @@ cudaError_t launch_noise_tables(ChainDev* d_chains, const NoiseTables& tb, int m
 cudaError_t launch_eta_ahead(const SysDev* sys, const int2* tiles, int ntiles, int max_blocks, cudaStream_t stream);
 // Blocks (one per SM) of the CG launch_cg would start for `a` (the step's
 // persistent CG on the real path).
-int cg_predict_grid(const CGArgs& a, bool mixed);
+int cg_predict_grid(const CGArgs& a, bool mixed, const OneLattice& lat);
 
 // Force + drift (+ per-tile max|drift| and sum F), then the Euler update and
 // observables (yk_langevin.cu).  mode 0: drift = F + bosonic drift;
