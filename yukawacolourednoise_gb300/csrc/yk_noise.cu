@@ -23,65 +23,115 @@
 
 namespace yk {
 
-// In-place FFT of `nseq` sequences of length N in shared memory; element j of
-// sequence c is buf[j * sj + c * sc].  Radix-2 for powers of two, direct DFT
-// (through tmp) otherwise.  tw[k] = exp(-2 pi i k / N), k < N.
-__device__ void smem_fft(double2* buf, double2* tmp, int N, int nseq, int sj, int sc,
-                         const double2* __restrict__ tw, bool inverse)
+__device__ __forceinline__ double2 c_add(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 c_sub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 c_mul(double2 a, double2 w)
 {
-    const int nt = blockDim.x;
-    if ((N & (N - 1)) == 0) {
-        int lg = 0;
-        while ((1 << lg) < N) ++lg;
-        for (int idx = threadIdx.x; idx < N * nseq; idx += nt) {
-            const int c = idx >> lg, j = idx & (N - 1);
-            const int rj = (int)(__brev((unsigned)j) >> (32 - lg));
-            if (lg > 0 && j < rj) {
-                double2* a = buf + j * sj + c * sc;
-                double2* b = buf + rj * sj + c * sc;
-                const double2 t = *a;
-                *a = *b;
-                *b = t;
-            }
-        }
-        __syncthreads();
-        for (int s = 1; s <= lg; ++s) {
-            const int h = 1 << (s - 1);   // butterfly span; twiddle stride N / 2^s
-            for (int idx = threadIdx.x; idx < (N >> 1) * nseq; idx += nt) {
-                const int c = idx >> (lg - 1), bidx = idx & ((N >> 1) - 1);
-                const int grp = bidx >> (s - 1), k = bidx & (h - 1);
-                const int i0 = (grp << s) + k, i1 = i0 + h;
-                double2 w = tw[k << (lg - s)];
-                if (inverse) w.y = -w.y;
-                double2* pa = buf + i0 * sj + c * sc;
-                double2* pb = buf + i1 * sj + c * sc;
-                const double2 u = *pa, v0 = *pb;
-                const double2 v = make_double2(v0.x * w.x - v0.y * w.y, v0.x * w.y + v0.y * w.x);
-                *pa = make_double2(u.x + v.x, u.y + v.y);
-                *pb = make_double2(u.x - v.x, u.y - v.y);
-            }
-            __syncthreads();
-        }
-    } else {
-        for (int idx = threadIdx.x; idx < N * nseq; idx += nt) {
-            const int c = idx / N, k = idx - c * N;
-            double sr = 0.0, si = 0.0;
-            for (int j = 0; j < N; ++j) {
-                double2 w = tw[(int)(((long long)j * k) % N)];
-                if (inverse) w.y = -w.y;
-                const double2 x = buf[j * sj + c * sc];
-                sr += x.x * w.x - x.y * w.y;
-                si += x.x * w.y + x.y * w.x;
-            }
-            tmp[k * sj + c * sc] = make_double2(sr, si);
-        }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < N * nseq; idx += nt) {
-            const int c = idx / N, j = idx - c * N;
-            buf[j * sj + c * sc] = tmp[j * sj + c * sc];
-        }
-        __syncthreads();
+    return make_double2(fma(a.x, w.x, -a.y * w.y), fma(a.x, w.y, a.y * w.x));
+}
+
+// A stage of the transform below: sub-sequences of r n points out of n ones
+// (m = n / r), s of them interleaved.  Butterfly b of a sequence takes elements
+// b + j M (M = N / r); with b = p s + q its outputs, times w_n^{p k}, go to q + s (r p + k).
+struct FftStage {
+    const double2* x;
+    double2* y;
+    int N, M, s, sj, sc, nseq;
+    bool twiddle, inverse;
+    const double2* tw;
+
+    __device__ __forceinline__ double2 in(int b, int j, int c) const { return x[(b + j * M) * sj + c * sc]; }
+    __device__ __forceinline__ double2 root(int k) const   // exp(-+2 pi i k / N), k < N
+    {
+        double2 w = tw[k];
+        if (inverse) w.y = -w.y;
+        return w;
     }
+    // output k of a butterfly
+    __device__ __forceinline__ void out(int p, int q, int r, int k, int c, double2 v) const
+    {
+        if (twiddle && k > 0) v = c_mul(v, root(p * k * s));
+        y[(q + s * (r * p + k)) * sj + c * sc] = v;
+    }
+};
+
+__device__ __forceinline__ void fft_even(const FftStage& f, int r)   // r = 4 or 2
+{
+    for (int idx = threadIdx.x; idx < f.M * f.nseq; idx += blockDim.x) {
+        const int c = idx / f.M, b = idx - c * f.M, p = b / f.s, q = b - p * f.s;
+        const double2 a0 = f.in(b, 0, c), a1 = f.in(b, 1, c);
+        if (r == 4) {
+            const double2 a2 = f.in(b, 2, c), a3 = f.in(b, 3, c);
+            const double2 t0 = c_add(a0, a2), t1 = c_sub(a0, a2), t2 = c_add(a1, a3), d = c_sub(a1, a3);
+            const double2 t3 = f.inverse ? make_double2(-d.y, d.x) : make_double2(d.y, -d.x);
+            f.out(p, q, 4, 0, c, c_add(t0, t2));
+            f.out(p, q, 4, 1, c, c_add(t1, t3));
+            f.out(p, q, 4, 2, c, c_sub(t0, t2));
+            f.out(p, q, 4, 3, c, c_sub(t1, t3));
+        } else {
+            f.out(p, q, 2, 0, c, c_add(a0, a1));
+            f.out(p, q, 2, 1, c, c_sub(a0, a1));
+        }
+    }
+}
+
+// Outputs k and r - k of an odd r share their sums over a_j + a_{r-j} and a_j - a_{r-j}.
+__device__ __forceinline__ void fft_odd(const FftStage& f, int r)
+{
+    const int h = r / 2, items = f.M * (h + 1);
+    for (int idx = threadIdx.x; idx < items * f.nseq; idx += blockDim.x) {
+        const int c = idx / items, e = idx - c * items, k = e / f.M, b = e - k * f.M, p = b / f.s, q = b - p * f.s;
+        double2 R = f.in(b, 0, c), I = make_double2(0.0, 0.0);
+        int t = 0;   // j k mod r
+        for (int j = 1; j <= h; ++j) {
+            t += k;
+            if (t >= r) t -= r;
+            const double2 u = f.in(b, j, c), v = f.in(b, r - j, c), w = f.root(t * f.M);
+            const double2 S = c_add(u, v), D = c_sub(u, v);
+            R.x = fma(w.x, S.x, R.x);
+            R.y = fma(w.x, S.y, R.y);
+            I.x = fma(-w.y, D.y, I.x);   // i sin D
+            I.y = fma(w.y, D.x, I.y);
+        }
+        f.out(p, q, r, k, c, c_add(R, I));
+        if (k > 0) f.out(p, q, r, r - k, c, c_sub(R, I));
+    }
+}
+
+// FFT of `nseq` sequences of length N in shared memory; element j of sequence c
+// is buf[j * sj + c * sc].  Radix 4, 2 and every odd prime of N, each stage from
+// one of the two buffers into the other (self-sorting); returns the one that
+// holds the result.  tw[k] = exp(-2 pi i k / N), k < N.  Bound by the FP64 pipe:
+// a prime r costs about 4 r operations a point, so that a length with small
+// factors is far from a direct sum's 4 N (the noise of a 160 x 224 step in all:
+// 291 us by direct sums, 53 so).
+__device__ double2* smem_fft(double2* buf, double2* tmp, int N, int nseq, int sj, int sc,
+                             const double2* __restrict__ tw, bool inverse)
+{
+    int n = N, s = 1, prime = 3;
+    while (n > 1) {
+        int r;
+        if (n % 4 == 0) {
+            r = 4;
+        } else if (n % 2 == 0) {
+            r = 2;
+        } else {
+            while (n % prime) prime = prime * prime > n ? n : prime + 2;
+            r = prime;
+        }
+        const FftStage f = {buf, tmp, N, N / r, s, sj, sc, nseq, n > r, inverse, tw};
+        if (r & 1)
+            fft_odd(f, r);
+        else
+            fft_even(f, r);
+        __syncthreads();
+        n /= r;
+        s *= r;
+        double2* const q = buf;
+        buf = tmp;
+        tmp = q;
+    }
+    return buf;
 }
 
 __device__ __forceinline__ double white_at(const ChainDev& C, const double* given, int n)
@@ -124,7 +174,7 @@ __global__ void __launch_bounds__(kBlock) noise_rows_fwd(ChainDev* chains, const
             buf[x] = make_double2(white_at(C, given, base + x), two ? white_at(C, given, base + Nx + x) : 0.0);
     }
     __syncthreads();
-    smem_fft(buf, tmp, Nx, 1, 1, 0, C.tw_x, false);
+    buf = smem_fft(buf, tmp, Nx, 1, 1, 0, C.tw_x, false);
     for (int k = threadIdx.x; k < Nx; k += blockDim.x) {
         if (!C.keep[k]) continue;   // the column keeps no mode
         const double2 zk = buf[k], zm = buf[k == 0 ? 0 : Nx - k];
@@ -151,7 +201,10 @@ __global__ void __launch_bounds__(kBlock) noise_cols(ChainDev* chains, const int
         buf[idx] = C.keep[x0 + c] ? C.spec[t * Nx + x0 + c] : make_double2(0.0, 0.0);   // unwritten otherwise
     }
     __syncthreads();
-    smem_fft(buf, tmp, Nt, cw, cw, 1, C.tw_t, false);
+    if (double2* const q = smem_fft(buf, tmp, Nt, cw, cw, 1, C.tw_t, false); q != buf) {
+        tmp = buf;
+        buf = q;
+    }
     const double inv = 1.0 / (double)C.V;
     for (int idx = threadIdx.x; idx < Nt * cw; idx += blockDim.x) {
         const int t = idx / cw, c = idx - t * cw;
@@ -160,7 +213,7 @@ __global__ void __launch_bounds__(kBlock) noise_cols(ChainDev* chains, const int
         buf[idx].y *= m;
     }
     __syncthreads();
-    smem_fft(buf, tmp, Nt, cw, cw, 1, C.tw_t, true);
+    buf = smem_fft(buf, tmp, Nt, cw, cw, 1, C.tw_t, true);
     for (int idx = threadIdx.x; idx < Nt * cw; idx += blockDim.x) {
         const int t = idx / cw, c = idx - t * cw;
         C.spec[t * Nx + x0 + c] = buf[idx];
@@ -192,7 +245,7 @@ __global__ void __launch_bounds__(kBlock) noise_rows_inv(ChainDev* chains, const
         buf[x] = v;
     }
     __syncthreads();
-    smem_fft(buf, tmp, Nx, 1, 1, 0, C.tw_x, true);
+    buf = smem_fft(buf, tmp, Nx, 1, 1, 0, C.tw_x, true);
     for (int x = threadIdx.x; x < Nx; x += blockDim.x) {
         C.xi[t * Nx + x] = buf[x].x;
         if (two) C.xi[(t + 1) * Nx + x] = buf[x].y;
