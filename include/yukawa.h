@@ -375,11 +375,14 @@ typedef struct yk_profile {
     int launches;                /* kernels launched by those steps               */
     int cg_launches;             /* persistent CG launches                        */
     int cg_grid;                 /* blocks of the last CG launch                  */
-    int cg_kernel;               /* its kernel: 0 grid-wide, 1 halo, 2 cluster,   */
-                                 /*   3 even-odd (Schur complement), 4 batched    */
-                                 /*   even-odd (work dealt out per pass), 5       */
-                                 /*   batched even-odd over 32 x 16 patches, 6    */
-                                 /*   a cluster per system (small FP64 lattices)  */
+    int cg_kernel;               /* its form: D^dag D by 0 the grid-wide kernel,  */
+                                 /*   1 halos, 2 a cluster (opt-in), 6 a cluster  */
+                                 /*   per system (small FP64 lattices); even-odd  */
+                                 /*   (Schur complement) of 3 one system, 4 a     */
+                                 /*   batch, 5 a batch that 32 x 16 patches tile: */
+                                 /*   on a cluster per system where all fit one   */
+                                 /*   (cg_grid: the clusters' blocks), else on    */
+                                 /*   the whole GPU                               */
     double noise_ms, cg_ms, force_ms, update_ms;   /* summed device time          */
     int64_t cg_iterations;       /* CG iterations, summed over systems            */
     int64_t cg_site_iterations;  /* sum over chains of iterations x volume        */

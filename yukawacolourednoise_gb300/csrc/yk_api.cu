@@ -97,6 +97,15 @@ struct Chain {
     double *peta = nullptr, *ptile = nullptr, *ptile_f = nullptr;
 };
 
+constexpr int kEocLanes = 4;      // parallel branches of the cluster-resident solves
+constexpr int kEocSpread = 16;    // a system takes up to that many times the fewest CTAs
+constexpr int kEocCtas = 128;     // while all systems together take no more than this
+
+struct EocGroup {
+    int first, count;   // its systems in d_eoc_order
+    EocForm form;
+};
+
 }  // namespace
 
 struct yk_ctx {
@@ -205,6 +214,14 @@ struct yk_ctx {
     int2* d_eo_tiles = nullptr;
     int eo_tile_begin = 0, eo_tile_end = 0;
     bool eo_patches = false;   // every system tiled by 32 x 16 patches of its compact lattice
+    // the step's solves by cg_eoc_kernel (empty: not taken): groups of systems of
+    // one form, their systems in d_eoc_order, launched on parallel branches
+    // (eoc_parallel; else one after another: the autotuner's choice)
+    std::vector<EocGroup> eoc;
+    int* d_eoc_order = nullptr;
+    bool eoc_parallel = true;
+    cudaStream_t eoc_lane[kEocLanes] = {};   // lane 0 is the stream itself
+    cudaEvent_t eoc_fork = nullptr, eoc_join[kEocLanes] = {};
 };
 
 namespace {
@@ -405,23 +422,71 @@ OneLattice step_lattice(const yk_ctx* ctx)
     return q;
 }
 
+// What the step's solves by cg_eoc_kernel start from.
+int prepare_step_eoc(yk_ctx* ctx, const CGArgs& a)
+{
+    bool r1 = false, other = false;
+    int nh = 0;
+    for (const EocGroup& G : ctx->eoc) {
+        (G.form.r1 ? r1 : other) = true;
+        nh = std::max(nh, G.form.nh);
+    }
+    YK_CK(launch_eoc_prepare(a, r1, other, nh, ctx->stream));
+    return YK_OK;
+}
+
+// The step's solves by cg_eoc_kernel: its groups of one form, the largest
+// clusters first, on parallel branches -- a group's clusters start as the ones
+// before it leave SMs, instead of after their last.
+int launch_step_eoc(yk_ctx* ctx, const CGArgs& a)
+{
+    const int n = ctx->eoc_parallel ? std::min((int)ctx->eoc.size(), kEocLanes) : 1;
+    if (n > 1) {
+        YK_CK(cudaEventRecord(ctx->eoc_fork, ctx->stream));
+        for (int i = 1; i < n; ++i) YK_CK(cudaStreamWaitEvent(ctx->eoc_lane[i], ctx->eoc_fork, 0));
+    }
+    for (size_t g = 0; g < ctx->eoc.size(); ++g) {
+        const int i = (int)(g % n);
+        const EocGroup& G = ctx->eoc[g];
+        YK_CK(launch_cg_eoc(a, G.form, ctx->d_eoc_order + G.first, G.count, i ? ctx->eoc_lane[i] : ctx->stream));
+    }
+    for (int i = 1; i < n; ++i) {
+        YK_CK(cudaEventRecord(ctx->eoc_join[i], ctx->eoc_lane[i]));
+        YK_CK(cudaStreamWaitEvent(ctx->stream, ctx->eoc_join[i], 0));
+    }
+    return YK_OK;
+}
+
+// Blocks of the step's CG.
+int step_cg_grid(yk_ctx* ctx)
+{
+    if (ctx->eoc.empty()) return cg_predict_grid(step_cg_args(ctx), ctx->precision == YK_MIXED, step_lattice(ctx));
+    int n = 0;
+    for (const EocGroup& G : ctx->eoc) n += G.form.c * G.count;
+    return n;
+}
+
 int enqueue_step(yk_ctx* ctx)
 {
     cudaEvent_t e = nullptr;
     NoiseTables nt = {ctx->d_rows, ctx->nrows, ctx->d_cols, ctx->ncols, ctx->d_white, ctx->nwhite};
     int free_sm = 0;
     if (ctx->noise_overlap && !ctx->profiling && !ctx->cg_cluster && ctx->nsys > 0 && ctx->nrows > 0)
-        free_sm = ctx->n_sm - cg_predict_grid(step_cg_args(ctx), ctx->precision == YK_MIXED, step_lattice(ctx));
+        free_sm = ctx->n_sm - step_cg_grid(ctx);
     const bool overlap = free_sm >= 8 && ctx->overlap_choice != 0;
-    if (overlap) {
-        YK_CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
+    auto beside = [&]() -> int {
         YK_CK(cudaStreamWaitEvent(ctx->aux, ctx->fork_ev, 0));
         YK_CK(launch_noise_tables(ctx->d_chains, nt, ctx->max_nx, ctx->max_cols, nullptr, ctx->aux, free_sm));
         YK_CK(cudaEventRecord(ctx->join_ev, ctx->aux));
         // the next step's sources, which its CG would otherwise generate first
         YK_CK(launch_eta_ahead(ctx->d_sys, ctx->d_sys_tiles, ctx->n_sys_tiles, free_sm, ctx->aux));
         YK_CK(cudaEventRecord(ctx->join2_ev, ctx->aux));
-    } else {
+        return YK_OK;
+    };
+    if (overlap && ctx->eoc.empty()) {
+        YK_CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
+        if (int rc = beside()) return rc;
+    } else if (!overlap) {
         prof_begin(ctx, &e);
         YK_CK(launch_noise_tables(ctx->d_chains, nt, ctx->max_nx, ctx->max_cols, nullptr, ctx->stream));
         prof_end(ctx, 0, e, (ctx->nwhite > 0 ? 1 : 0) + (ctx->nrows > 0 ? 3 : 0));
@@ -435,6 +500,18 @@ int enqueue_step(yk_ctx* ctx)
             ctx->cg_grid = 16 * ctx->nsys;
             ctx->cg_kernel = 2;
             prof_end(ctx, 1, e, 2);
+        } else if (!ctx->eoc.empty()) {
+            if (int rc = prepare_step_eoc(ctx, a)) return rc;
+            if (overlap) YK_CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
+            if (int rc = launch_step_eoc(ctx, a)) return rc;
+            // the noise after the clusters in the order of the launches: its blocks
+            // spread over every GPC, and a cluster of 16 that came second would wait
+            // for them to leave one (160 x 224: 437 us a step against 317)
+            if (overlap)
+                if (int rc = beside()) return rc;
+            ctx->cg_grid = step_cg_grid(ctx);
+            ctx->cg_kernel = ctx->nsys == 1 ? 3 : ctx->eo_patches ? 5 : 4;
+            prof_end(ctx, 1, e, (int)ctx->eoc.size() + 1);
         } else {
             // batched: block ranges balanced by the previous step's iterations
             const bool bal = ctx->nsys > 1 && ctx->cg_balance && !ctx->cg_eo;
@@ -633,9 +710,13 @@ int chain_solve(yk_ctx* ctx, int c, int kind, yk_solve_stats* stats, bool want_x
         a.solo_nx = C.Nx;
     }
     if (!want_x) eo_args(ctx, a);
+    EocForm form;
     if (ctx->cg_cluster) {
         YK_CK(launch_eta(ctx->d_sys, ctx->d_sys_tiles + C.cg_tile0, C.cg_tile1 - C.cg_tile0, kind, ctx->stream));
         YK_CK(launch_cg_cluster(a, ctx->cluster_sites, ctx->stream));
+    } else if (a.sys_eo && !ctx->eoc.empty() && cg_eoc_form(C.Nt, C.Nx / 2, C.a.r, kEocSpread, &form)) {
+        YK_CK(launch_eoc_prepare(a, form.r1, !form.r1, form.nh, ctx->stream));
+        YK_CK(launch_cg_eoc(a, form, nullptr, C.n_rhs_step, ctx->stream));
     } else {
         YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, nullptr, nullptr, {C.Nt, C.Nx, 0}));
     }
@@ -674,7 +755,7 @@ int tune_overlap(yk_ctx* ctx)
 {
     yk_tune_result& T = ctx->tune;
     if (!ctx->noise_overlap || ctx->cg_cluster || ctx->nsys == 0 || ctx->nrows == 0 || ctx->pions) return YK_OK;
-    if (ctx->n_sm - cg_predict_grid(step_cg_args(ctx), ctx->precision == YK_MIXED, step_lattice(ctx)) < 8) return YK_OK;
+    if (ctx->n_sm - step_cg_grid(ctx) < 8) return YK_OK;
     const int nch = (int)ctx->ch.size();
     size_t nphi = 0;
     for (const Chain& C : ctx->ch) nphi += (size_t)C.V;
@@ -748,7 +829,42 @@ int run_autotune(yk_ctx* ctx)
     yk_tune_result& T = ctx->tune;
     T = yk_tune_result{};
     const bool mixed = ctx->precision == YK_MIXED;
-    if (ctx->nsys > 1 && !ctx->cg_cluster) {
+    if (ctx->eoc.size() > 1) {
+        // cluster-resident solves: their groups on parallel branches or one after
+        // another, timed over the step's CG (one warm-up, two launches)
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        YK_CK(cudaEventCreate(&e0));
+        YK_CK(cudaEventCreate(&e1));
+        CGArgs a = step_cg_args(ctx);
+        a.eta_kind = 100;
+        a.max_iter = std::min(ctx->max_iter, 48);
+        float ms[2] = {0.f, 0.f};
+        int rc = YK_OK;
+        cudaError_t e = cudaSuccess;
+        for (int cand = 1; cand >= 0 && rc == YK_OK && e == cudaSuccess; --cand) {
+            ctx->eoc_parallel = cand != 0;
+            rc = prepare_step_eoc(ctx, a);
+            if (rc == YK_OK) rc = launch_step_eoc(ctx, a);
+            if (rc == YK_OK) e = cudaEventRecord(e0, ctx->stream);
+            for (int rep = 0; rep < 2 && rc == YK_OK && e == cudaSuccess; ++rep) rc = launch_step_eoc(ctx, a);
+            if (rc == YK_OK && e == cudaSuccess) e = cudaEventRecord(e1, ctx->stream);
+            if (rc == YK_OK && e == cudaSuccess) e = cudaEventSynchronize(e1);
+            if (rc == YK_OK && e == cudaSuccess) e = cudaEventElapsedTime(&ms[cand], e0, e1);
+            if (rc == YK_OK && e == cudaSuccess) rc = status_of_err(ctx);
+        }
+        cudaEventDestroy(e0);
+        cudaEventDestroy(e1);
+        if (rc) return rc;
+        if (e != cudaSuccess) {
+            set_error("autotune: %s", cudaGetErrorString(e));
+            return YK_ECUDA;
+        }
+        ctx->eoc_parallel = ms[1] <= ms[0];
+        T.cg_candidates = 2;
+        T.cg_grid = T.cg_grid_max = step_cg_grid(ctx);
+        T.cg_ms_chosen = std::min(ms[0], ms[1]);
+        T.cg_ms_max = std::max(ms[0], ms[1]);
+    } else if (ctx->nsys > 1 && !ctx->cg_cluster && ctx->eoc.empty()) {
         const int maxg = ctx->cg_eo ? cg_eob_max_grid() : cg_max_grid(1, mixed);
         std::vector<int> cand = {maxg, maxg * 3 / 4, maxg / 2, ctx->n_sm, ctx->n_sm / 2};
         std::sort(cand.begin(), cand.end(), std::greater<int>());
@@ -889,6 +1005,59 @@ int pion_setup(yk_ctx* ctx)
     return YK_OK;
 }
 
+// The step's solves as groups of cg_eoc_kernel, when every system fits a cluster.
+// The systems spread over more CTAs than they need while all of them still find
+// SMs at once (kEocCtas: eight GPCs' clusters of 16): a lone small system is
+// bound by the latency of a CTA's passes, a batch by its SMs' throughput, where
+// the fewest CTAs a system (the least work on edge rows) is best.
+// YK_CG_EOC=0, or YK_CG_EO_PATCH / YK_CG_EOP, which choose among the other
+// even-odd kernels, turn this off.
+int eoc_setup(yk_ctx* ctx, const std::vector<SysDev>& views)
+{
+    const char* env = getenv("YK_CG_EOC");
+    if ((env && env[0] == '0') || getenv("YK_CG_EO_PATCH") || getenv("YK_CG_EOP")) return YK_OK;
+    std::vector<EocForm> form(views.size());
+    for (int spread = kEocSpread;; spread /= 2) {
+        int ctas = 0;
+        for (size_t q = 0; q < views.size(); ++q) {
+            if (!cg_eoc_form(views[q].Nt, views[q].Nx, views[q].r, spread, &form[q])) return YK_OK;
+            ctas += form[q].c;
+        }
+        if (ctas <= kEocCtas || spread == 1) break;
+    }
+    std::vector<int> order(views.size());
+    for (size_t q = 0; q < order.size(); ++q) order[q] = (int)q;
+    // the same order whatever the run: by cluster size (largest first), then by the
+    // rest of the form, then by the system
+    auto key = [&](int q) { return std::make_tuple(-form[q].c, -form[q].u, !form[q].r1, !form[q].full); };
+    std::stable_sort(order.begin(), order.end(), [&](int l, int r) { return key(l) < key(r); });
+    std::vector<EocGroup> groups;
+    for (size_t i = 0; i < order.size(); ++i) {
+        const EocForm& f = form[order[i]];
+        EocForm both = f;   // one shared-memory layout serves the group's lattices while it fits
+        if (i > 0) {
+            both.cells = std::max(f.cells, groups.back().form.cells);
+            both.nh = std::max(f.nh, groups.back().form.nh);
+        }
+        if (i == 0 || key(order[i]) != key(order[i - 1]) || eoc_smem(both) > kEocMaxSmem)
+            groups.push_back({(int)i, 0, f});
+        else
+            groups.back().form = both;
+        ++groups.back().count;
+    }
+    YK_CK(cudaMalloc(&ctx->d_eoc_order, sizeof(int) * order.size()));
+    YK_CK(cudaMemcpy(ctx->d_eoc_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
+    if (groups.size() > 1) {
+        YK_CK(cudaEventCreateWithFlags(&ctx->eoc_fork, cudaEventDisableTiming));
+        for (int i = 1; i < std::min((int)groups.size(), kEocLanes); ++i) {
+            YK_CK(cudaStreamCreateWithFlags(&ctx->eoc_lane[i], cudaStreamNonBlocking));
+            YK_CK(cudaEventCreateWithFlags(&ctx->eoc_join[i], cudaEventDisableTiming));
+        }
+    }
+    ctx->eoc = std::move(groups);
+    return YK_OK;
+}
+
 // Compact (even-odd) views of the step's single mixed system: the lattice of
 // one parity class (Nx / 2 columns, V / 2 sites) over the system's buffers --
 // the FP32 vectors compact, x = chi_e followed by rhs_e, t64 the full chi at
@@ -942,6 +1111,7 @@ int eo_setup(yk_ctx* ctx, const std::vector<SysDev>& hs)
         ctx->eo_tile_begin = 0;
         ctx->eo_tile_end = ctx->n_sys_tiles;
     }
+    if (int rc = eoc_setup(ctx, views)) return rc;
     // every step system's compact lattice tiled by 32 x 16 patches: batches may
     // take the patch kernel
     ctx->eo_patches = true;
@@ -1058,6 +1228,7 @@ int yk_ctx_create(const yk_params* params, int n_chains, yk_ctx** out)
     cg_max_grid(2, true);
     if (mixed) cg_halo_init();
     cg_small_init();
+    if (mixed) cg_eoc_init();
     noise_init_attributes();
     {
         // opt-in while its FP64 reliable updates run on 16 SMs only
@@ -1408,6 +1579,12 @@ int yk_ctx_destroy(yk_ctx* ctx)
     if (ctx->mem) cudaFree(ctx->mem);
     if (ctx->pion_mem) cudaFree(ctx->pion_mem);
     if (ctx->eo_mem) cudaFree(ctx->eo_mem);
+    if (ctx->d_eoc_order) cudaFree(ctx->d_eoc_order);
+    for (cudaStream_t q : ctx->eoc_lane)
+        if (q) cudaStreamDestroy(q);
+    for (cudaEvent_t q : ctx->eoc_join)
+        if (q) cudaEventDestroy(q);
+    if (ctx->eoc_fork) cudaEventDestroy(ctx->eoc_fork);
     if (ctx->aux) {
         cudaStreamSynchronize(ctx->aux);
         cudaStreamDestroy(ctx->aux);

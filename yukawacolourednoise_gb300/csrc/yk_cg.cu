@@ -38,6 +38,7 @@
 #include <type_traits>
 
 #include "yk_common.cuh"
+#include "yk_ff.cuh"
 #include "yk_kernels.h"
 
 namespace yk {
@@ -158,75 +159,6 @@ __device__ __forceinline__ W pick(double d, float f)
 }
 
 // ---------------------------------------------------------------------------
-// Float-float sums (hi + lo, about 48 significant bits) for the mixed solver:
-// GB300 issues FP64 at 1/64 of the FP32 rate, so its reductions run on the
-// FP32 pipes.  Knuth's two-sum; no multiplications, so no FMA contraction.
-// ---------------------------------------------------------------------------
-struct FF {
-    float hi, lo;
-};
-
-__device__ __forceinline__ FF ff_add(FF a, FF b)
-{
-    const float s = a.hi + b.hi;
-    const float bp = s - a.hi;
-    float e = (a.hi - (s - bp)) + (b.hi - bp);
-    e += a.lo + b.lo;
-    const float hi = s + e;
-    return FF{hi, e - (hi - s)};
-}
-
-__device__ __forceinline__ FF ff_of(double x)
-{
-    const float hi = (float)x;
-    return FF{hi, (float)(x - (double)hi)};
-}
-
-__device__ __forceinline__ FF ff_shfl_xor(FF a, int o)
-{
-    return FF{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-}
-
-// Float-float products and the reciprocal (Dekker's product with the exact
-// FMA error term; one Newton step from the FP32 reciprocal).  The explicitly
-// rounded intrinsics keep the compiler from contracting the product that the
-// error term subtracts.
-__device__ __forceinline__ FF ff_renorm(float p, float e)
-{
-    const float hi = __fadd_rn(p, e);
-    return FF{hi, __fsub_rn(e, __fsub_rn(hi, p))};
-}
-
-__device__ __forceinline__ FF ff_mul(FF a, FF b)
-{
-    const float p = __fmul_rn(a.hi, b.hi);
-    float e = __fmaf_rn(a.hi, b.hi, -p);
-    e = __fmaf_rn(a.hi, b.lo, e);
-    e = __fmaf_rn(a.lo, b.hi, e);
-    return ff_renorm(p, e);
-}
-
-__device__ __forceinline__ FF ff_mul_f(FF a, float b)
-{
-    const float p = __fmul_rn(a.hi, b);
-    float e = __fmaf_rn(a.hi, b, -p);
-    e = __fmaf_rn(a.lo, b, e);
-    return ff_renorm(p, e);
-}
-
-__device__ __forceinline__ FF ff_sub(FF a, FF b) { return ff_add(a, FF{-b.hi, -b.lo}); }
-__device__ __forceinline__ double dbl_of(FF a) { return (double)a.hi + (double)a.lo; }
-
-// 1 / d: y = rn(1 / d.hi), then y + y (1 - d y) with d y and the correction in
-// float-float (relative error about 2^-47)
-__device__ __forceinline__ FF ff_rcp(FF d)
-{
-    const float y = __frcp_rn(d.hi);
-    const FF e = ff_sub(FF{1.f, 0.f}, ff_mul_f(d, y));
-    return ff_add(FF{y, 0.f}, ff_mul_f(e, y));
-}
-
-// ---------------------------------------------------------------------------
 // Fixed-point sums (mixed single-system solves, real path).  Each tile adds
 // round(x * 2^e) of its four values (|r|^2, |Ap|^2, <p,Ap>, <r,Ap>) with a
 // 64-bit integer atomic: integer addition is exact and associative, so the
@@ -313,18 +245,6 @@ __device__ __forceinline__ bool fix_to_ff(long long S, int e, FF& out)
     out = S < 0 ? FF{-hi, -lo} : FF{hi, lo};
     return true;
 }
-
-// float-float times float (Dekker's product through the FMA, then a fast two-sum)
-__device__ __forceinline__ FF ff_mul(FF a, float b)
-{
-    const float p = a.hi * b;
-    float err = fmaf(a.hi, b, -p);
-    err = fmaf(a.lo, b, err);
-    const float s = p + err;
-    return FF{s, err - (s - p)};
-}
-
-__device__ __forceinline__ FF ff_neg(FF a) { return FF{-a.hi, -a.lo}; }
 
 // tile slot of value c (|r|^2, |Ap|^2, <p,Ap> re, <r,Ap> re) on the real path
 __device__ __forceinline__ int fix_value_of_slot(int i)
@@ -2434,51 +2354,6 @@ __device__ __forceinline__ Site<float, 1> eo_sm(const float4* in, int j, int Nh,
                                         diag, r, sp, sm);
 }
 
-// The even-odd kernels' reliable updates, round 0 and reconstruction in
-// float-float (about 48 significant bits, on the FP32 pipes: GB300 issues
-// FP64 at 1/64 of the FP32 rate and these passes were bound by it).  chi_e,
-// rhs_e and the odd intermediate keep the FP64 vectors' 32 bytes a compact
-// site: four hi words, then four lo words; 1 / A_o keeps its 8 bytes as (hi,
-// lo).  Only the kernels read them; chi goes out to the force in FP64.
-struct SiteFF {
-    FF v[4];
-};
-
-__device__ __forceinline__ SiteFF ld_ff(const double* base, int m)
-{
-    const float4* p = reinterpret_cast<const float4*>(base) + 2 * (size_t)m;
-    const float4 h = p[0], l = p[1];
-    return SiteFF{{FF{h.x, l.x}, FF{h.y, l.y}, FF{h.z, l.z}, FF{h.w, l.w}}};
-}
-
-__device__ __forceinline__ void st_ff(double* base, int m, const SiteFF& s)
-{
-    float4* p = reinterpret_cast<float4*>(base) + 2 * (size_t)m;
-    p[0] = make_float4(s.v[0].hi, s.v[1].hi, s.v[2].hi, s.v[3].hi);
-    p[1] = make_float4(s.v[0].lo, s.v[1].lo, s.v[2].lo, s.v[3].lo);
-}
-
-__device__ __forceinline__ FF ld_ff1(const double* base, int m)
-{
-    const float2 v = reinterpret_cast<const float2*>(base)[m];
-    return FF{v.x, v.y};
-}
-
-__device__ __forceinline__ void st_ff1(double* base, int m, FF v)
-{
-    reinterpret_cast<float2*>(base)[m] = make_float2(v.hi, v.lo);
-}
-
-// a source vector's site as float-float: the Langevin sources are FP32 normals
-// (exact in FP32) when generated; other right-hand sides are split
-__device__ __forceinline__ SiteFF ff_site_of(const Site<double, 1>& e, bool exact32)
-{
-    SiteFF s;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) s.v[i] = exact32 ? FF{(float)e.v[i], 0.f} : ff_of(e.v[i]);
-    return s;
-}
-
 // dirac_combine's hop coefficients in float-float: P = -(r + 1) / 2,
 // M = -(r - 1) / 2, A = -r / 2 (the time hops take +-P and +-M by the
 // antiperiodic signs, the space hops A and +-1/2)
@@ -2498,8 +2373,6 @@ __device__ __forceinline__ HopFF hop_of_r(double r)
     const FF rp = ff_add(rr, FF{1.f, 0.f}), rm = ff_add(rr, FF{-1.f, 0.f});
     return HopFF{FF{-0.5f * rp.hi, -0.5f * rp.lo}, FF{-0.5f * rm.hi, -0.5f * rm.lo}, FF{-0.5f * rr.hi, -0.5f * rr.lo}};
 }
-
-__device__ __forceinline__ FF ff_sign(FF a, float s) { return FF{s * a.hi, s * a.lo}; }
 
 // dirac_combine<float-float, K = 1, DAG> with the same order of terms:
 // MODE 0: H alone; 1: c + H; 2: diag c + H

@@ -31,7 +31,7 @@
 #include <cfloat>
 #include <type_traits>
 
-#include "yk_common.cuh"
+#include "yk_cluster.cuh"
 #include "yk_kernels.h"
 
 namespace yk {
@@ -48,79 +48,6 @@ template <typename W, int K>
 struct __align__(16) Unit {
     W v[2 * K];
 };
-
-// A sum in the precision it is carried: FP64, or float-float for FP32 vectors.
-struct Sum2 {
-    float hi, lo;
-};
-
-__device__ __forceinline__ double s_add(double a, double b) { return a + b; }
-__device__ __forceinline__ Sum2 s_add(Sum2 a, Sum2 b)   // Knuth's two-sum with the low parts
-{
-    const float s = a.hi + b.hi, bp = s - a.hi;
-    float e = (a.hi - (s - bp)) + (b.hi - bp);
-    e += a.lo + b.lo;
-    const float hi = s + e;
-    return Sum2{hi, e - (hi - s)};
-}
-__device__ __forceinline__ double s_shfl(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
-__device__ __forceinline__ Sum2 s_shfl(Sum2 a, int o)
-{
-    return Sum2{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)};
-}
-__device__ __forceinline__ double s_val(double a) { return a; }
-__device__ __forceinline__ double s_val(Sum2 a) { return (double)a.hi + (double)a.lo; }
-__device__ __forceinline__ double s_of(double x, double) { return x; }
-__device__ __forceinline__ Sum2 s_of(double x, Sum2)
-{
-    const float hi = (float)x;
-    return Sum2{hi, (float)(x - (double)hi)};
-}
-__device__ __forceinline__ Sum2 s_of(float x, Sum2) { return Sum2{x, 0.f}; }
-__device__ __forceinline__ Sum2 s_of(Sum2 x, Sum2) { return x; }
-__device__ __forceinline__ double s_zero(double) { return 0.0; }
-__device__ __forceinline__ Sum2 s_zero(Sum2) { return Sum2{0.f, 0.f}; }
-
-// Sums four values over the warp: lane l returns value l >> 3.
-template <typename T>
-__device__ __forceinline__ T warp_sum4(const T (&v)[4])
-{
-    const int lane = threadIdx.x & 31;
-    const bool h = lane & 16, q = lane & 8;
-    const T a0 = s_add(h ? v[2] : v[0], s_shfl(h ? v[0] : v[2], 16));
-    const T a1 = s_add(h ? v[3] : v[1], s_shfl(h ? v[1] : v[3], 16));
-    T c = s_add(q ? a1 : a0, s_shfl(q ? a0 : a1, 8));
-    c = s_add(c, s_shfl(c, 4));
-    c = s_add(c, s_shfl(c, 2));
-    return s_add(c, s_shfl(c, 1));
-}
-
-__device__ __forceinline__ float warp_sum4(const float (&v)[4])
-{
-    const int lane = threadIdx.x & 31;
-    const bool h = lane & 16, q = lane & 8;
-    const unsigned full = 0xffffffffu;
-    const float a0 = (h ? v[2] : v[0]) + __shfl_xor_sync(full, h ? v[0] : v[2], 16);
-    const float a1 = (h ? v[3] : v[1]) + __shfl_xor_sync(full, h ? v[1] : v[3], 16);
-    float c = (q ? a1 : a0) + __shfl_xor_sync(full, q ? a0 : a1, 8);
-    c += __shfl_xor_sync(full, c, 4);
-    c += __shfl_xor_sync(full, c, 2);
-    return c + __shfl_xor_sync(full, c, 1);
-}
-
-__device__ __forceinline__ void cluster_barrier()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-// Generic address of a shared-memory location of this CTA in CTA `rank`.
-template <typename T>
-__device__ __forceinline__ T* in_cta(T* p, unsigned rank)
-{
-    T* q;
-    asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
-    return q;
-}
 
 // FP64 data of global memory that another CTA of the cluster wrote before the
 // last barrier: served by L2.
@@ -210,7 +137,7 @@ template <typename W, int K, int U>
 __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int pions)
 {
     constexpr bool MIXED = sizeof(W) == 4;
-    using T = typename std::conditional<MIXED, Sum2, double>::type;
+    using T = typename std::conditional<MIXED, FF, double>::type;
     using Un = Unit<W, K>;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     __shared__ T wred[kSmThreads / 32][4];

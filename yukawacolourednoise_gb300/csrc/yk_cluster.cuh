@@ -1,0 +1,69 @@
+// yk_cluster.cuh -- sums, barrier and remote shared memory of the solves that
+// run inside one thread-block cluster (yk_cg_small.cu, yk_cg_eoc.cu).
+#pragma once
+
+#include "yk_ff.cuh"
+
+namespace yk {
+
+// A sum in the precision it is carried: FP64, or float-float for FP32 vectors.
+__device__ __forceinline__ double s_add(double a, double b) { return a + b; }
+__device__ __forceinline__ FF s_add(FF a, FF b) { return ff_add(a, b); }
+__device__ __forceinline__ double s_shfl(double a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
+__device__ __forceinline__ FF s_shfl(FF a, int o) { return ff_shfl_xor(a, o); }
+__device__ __forceinline__ double s_val(double a) { return a; }
+__device__ __forceinline__ double s_val(FF a) { return (double)a.hi + (double)a.lo; }
+__device__ __forceinline__ double s_of(double x, double) { return x; }
+__device__ __forceinline__ FF s_of(double x, FF)
+{
+    const float hi = (float)x;
+    return FF{hi, (float)(x - (double)hi)};
+}
+__device__ __forceinline__ FF s_of(float x, FF) { return FF{x, 0.f}; }
+__device__ __forceinline__ FF s_of(FF x, FF) { return x; }
+__device__ __forceinline__ double s_zero(double) { return 0.0; }
+__device__ __forceinline__ FF s_zero(FF) { return FF{0.f, 0.f}; }
+
+// Sums four values over the warp: lane l returns value l >> 3.
+template <typename T>
+__device__ __forceinline__ T warp_sum4(const T (&v)[4])
+{
+    const int lane = threadIdx.x & 31;
+    const bool h = lane & 16, q = lane & 8;
+    const T a0 = s_add(h ? v[2] : v[0], s_shfl(h ? v[0] : v[2], 16));
+    const T a1 = s_add(h ? v[3] : v[1], s_shfl(h ? v[1] : v[3], 16));
+    T c = s_add(q ? a1 : a0, s_shfl(q ? a0 : a1, 8));
+    c = s_add(c, s_shfl(c, 4));
+    c = s_add(c, s_shfl(c, 2));
+    return s_add(c, s_shfl(c, 1));
+}
+
+__device__ __forceinline__ float warp_sum4(const float (&v)[4])
+{
+    const int lane = threadIdx.x & 31;
+    const bool h = lane & 16, q = lane & 8;
+    const unsigned full = 0xffffffffu;
+    const float a0 = (h ? v[2] : v[0]) + __shfl_xor_sync(full, h ? v[0] : v[2], 16);
+    const float a1 = (h ? v[3] : v[1]) + __shfl_xor_sync(full, h ? v[1] : v[3], 16);
+    float c = (q ? a1 : a0) + __shfl_xor_sync(full, q ? a0 : a1, 8);
+    c += __shfl_xor_sync(full, c, 4);
+    c += __shfl_xor_sync(full, c, 2);
+    return c + __shfl_xor_sync(full, c, 1);
+}
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    __syncwarp();   // the aligned forms below want the warp converged
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Generic address of a shared-memory location of this CTA in CTA `rank`.
+template <typename T>
+__device__ __forceinline__ T* in_cta(T* p, unsigned rank)
+{
+    T* q;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(q) : "l"(p), "r"(rank));
+    return q;
+}
+
+}  // namespace yk

@@ -18,7 +18,7 @@ namespace yk {
 constexpr int kBlock = 256;   // threads per block of the site kernels
 constexpr int kTile = 256;    // lattice sites per tile (one per thread)
 constexpr int kMaxFFT = 4096; // longest FFT edge handled in shared memory
-constexpr int kMaxDFT = 256;  // longest non-power-of-two edge (direct DFT)
+constexpr int kMaxDFT = 256;  // longest non-power-of-two edge
 constexpr int kMaxTilesPerBlock = 4096;  // tiles one CG block may own
 constexpr int kMaxGrid = 2048;           // blocks of a CG launch (neighbour flags allocated)
 constexpr int kEobMaxSystems = 1024;     // systems of one batched even-odd solve
@@ -94,7 +94,8 @@ struct CGState {
     int status;
     int n_ru;            // reliable updates (mixed)
     int mode;            // the system's mode in the pass that follows
-    int chi_ready;       // the solve ended in a reliable update: t64 holds D_first x of the final x
+    int chi_ready;       // 1: t64 holds D_first x of the final x; 2 (cg_eoc_kernel): its even sites are
+                         //   in x, its odd ones less A_o^-1 eta_o in t64, both compact SiteFF
 };
 
 // Per-system coefficients of the next pass (alpha: x += alpha p, r -= alpha A p;
@@ -155,6 +156,30 @@ struct OneLattice {
     int Nt, Nx;
     int pions;   // whether they carry pions
 };
+
+// How cg_eoc_kernel (yk_cg_eoc.cu) runs a system: c CTAs a cluster, up to u rows
+// a thread, nh compact columns, buffers of `cells` cells (a group of lattices:
+// the largest of each).
+struct EocForm {
+    int c, u, cells, nh;
+    bool r1;     // Wilson r = 1
+    bool full;   // every thread that owns rows owns u
+};
+constexpr size_t kEocMaxSmem = 224 * 1024;
+// Its shared memory: what the updates' first two buffers and the iterations share
+// (two halos of four rows; for each of the 512 threads 2 u + 4 parts of 8 bytes at
+// r = 1, of 16 else with u = 4, and 2 u floats), in cells of 16 bytes; then two
+// buffers, two halos, and A_e and 1 / A_o as pairs on the buffers' rows but four, and
+// two.
+inline int eoc_first_cells(const EocForm& f)
+{
+    const int it = 8 * f.nh + (f.r1 ? 512 * (2 * f.u + 4) / 2 + 512 * 2 * f.u / 4 : 512 * 12 + 512 * 2);
+    return it > 2 * f.cells ? it : 2 * f.cells;
+}
+inline size_t eoc_smem(const EocForm& f)
+{
+    return 16 * ((size_t)eoc_first_cells(f) + 2 * f.cells + 8 * f.nh) + 16 * (f.cells - 3 * (size_t)f.nh);
+}
 
 // Per-chain device record of the Langevin step.
 struct ChainDev {

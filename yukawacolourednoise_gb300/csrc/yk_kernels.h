@@ -28,6 +28,16 @@ cudaError_t launch_cg(const CGArgs& a, int K, bool mixed, cudaStream_t stream, i
 int cg_small_grid(const CGArgs& a, int K, bool mixed, const OneLattice& lat);
 cudaError_t launch_cg_small(const CGArgs& a, int K, bool mixed, const OneLattice& lat, cudaStream_t stream);
 void cg_small_init();
+// The even-odd solve of the step inside one cluster per system (yk_cg_eoc.cu):
+// the form of an Nt x Nh compact lattice (false: it does not fit), spread over up
+// to `spread` times the fewest CTAs; the launch for `count` systems of one form,
+// order[0 .. count) or, order null, from a.sys_first on (a as for launch_cg with
+// its compact views given); before it what the solves of a's tiles start from, for
+// systems of r = 1 and others, the widest of max_nh columns; the kernels' attributes (before any capture).
+bool cg_eoc_form(int Nt, int Nh, double r, int spread, EocForm* f);
+cudaError_t launch_cg_eoc(const CGArgs& a, const EocForm& f, const int* order, int count, cudaStream_t stream);
+cudaError_t launch_eoc_prepare(const CGArgs& a, bool r1, bool other, int max_nh, cudaStream_t stream);
+void cg_eoc_init();
 // Work-balanced block ranges (CGArgs::balance) for the next solve of the
 // systems of `a`, from their iteration counts in the solve just finished;
 // grid: the grid of that solve's launch.  No-op for a single system.

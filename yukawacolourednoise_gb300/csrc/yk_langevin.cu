@@ -19,7 +19,7 @@
 //   observables, advances Langevin time and the Philox step counter on the
 //   device, so the host never waits for eps (the reference copies eps to the
 //   host every step, main.cu:378-381).
-#include "yk_common.cuh"
+#include "yk_ff.cuh"
 #include "yk_kernels.h"
 
 namespace yk {
@@ -44,7 +44,20 @@ __global__ void __launch_bounds__(kTile) force_drift_kernel(StepArgs s, const Sy
             for (int j = 0; j < C.n_rhs; ++j) {
                 const SysDev& S = sys[C.sys0 + j];
                 Site<double, K> chi;
-                if (st && st[C.sys0 + j].chi_ready) {
+                const int ready = st ? st[C.sys0 + j].chi_ready : 0;
+                if (K == 1 && ready == 2) {
+                    // an even lattice's site n is compact site n / 2 of its class
+                    const bool odd = (n / C.Nx + n) & 1;
+                    SiteFF c = ld_ff(odd ? S.t64 : S.x, n >> 1);
+                    if (odd) {
+                        const FF inv = ff_rcp(ff_split(diag));
+                        const SiteFF e = ff_site_of(load_site<double, 1>(S.b, n), S.gen_eta != 0);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) c.v[q] = ff_add(ff_mul(e.v[q], inv), c.v[q]);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) chi.v[q * K] = widen(c.v[q].hi) + widen(c.v[q].lo);
+                } else if (ready) {
                     chi = load_site<double, K>(S.t64, n);
                 } else {
                     const Site<double, K> c = load_site<double, K>(S.x, n);
