@@ -43,12 +43,6 @@ constexpr int kSmThreads = 512;
 constexpr size_t kSmMaxSmem = 220 * 1024;
 constexpr int kSmMaxReal = 12288;   // sites of a real FP64 solve
 
-// One flavour of a site: u planes, then d planes.
-template <typename W, int K>
-struct __align__(16) Unit {
-    W v[2 * K];
-};
-
 // FP64 data of global memory that another CTA of the cluster wrote before the
 // last barrier: served by L2.
 template <int K>
@@ -105,19 +99,6 @@ __device__ __forceinline__ Unit<W, K> unit_dirac(const At& at, int i, const Hop&
         }
     }
     return o;
-}
-
-// The pion term of flavour f (pion_add, yk_common.cuh): s1..s3 = +-g pi,
-// c this flavour's entries, e the other's.
-template <typename W>
-__device__ __forceinline__ void unit_pions(Unit<W, 2>& o, const Unit<W, 2>& c, const Unit<W, 2>& e, int f, W s1, W s2,
-                                           W s3)
-{
-    const W q = f ? s2 : -s2, z = f ? -s3 : s3;
-    o.v[0] += fma(z, c.v[2], fma(s1, e.v[2], -q * e.v[3]));
-    o.v[1] += fma(z, c.v[3], fma(s1, e.v[3], q * e.v[2]));
-    o.v[2] -= fma(z, c.v[0], fma(s1, e.v[0], -q * e.v[1]));
-    o.v[3] -= fma(z, c.v[1], fma(s1, e.v[1], q * e.v[0]));
 }
 
 enum SmMode { kSmStep = 1, kSmRu = 2, kSmRedo = 3, kSmDone = 4 };

@@ -181,6 +181,25 @@ __device__ __forceinline__ void pion_term(Site<R, K>& o, const Site<R, K>& c, co
     }
 }
 
+// One flavour of a site: u planes, then d planes.
+template <typename W, int K>
+struct __align__(16) Unit {
+    W v[2 * K];
+};
+
+// The pion term of flavour f (pion_add, yk_common.cuh): s1..s3 = +-g pi,
+// c this flavour's entries, e the other's.
+template <typename W>
+__device__ __forceinline__ void unit_pions(Unit<W, 2>& o, const Unit<W, 2>& c, const Unit<W, 2>& e, int f, W s1, W s2,
+                                           W s3)
+{
+    const W q = f ? s2 : -s2, z = f ? -s3 : s3;
+    o.v[0] += fma(z, c.v[2], fma(s1, e.v[2], -q * e.v[3]));
+    o.v[1] += fma(z, c.v[3], fma(s1, e.v[3], q * e.v[2]));
+    o.v[2] -= fma(z, c.v[0], fma(s1, e.v[0], -q * e.v[1]));
+    o.v[3] -= fma(z, c.v[1], fma(s1, e.v[1], q * e.v[0]));
+}
+
 // ---------------------------------------------------------------------------
 // Philox4x32-10 (J. Salmon et al., "Parallel random numbers: as easy as
 // 1, 2, 3", SC'11) with the framework's counter scheme:

@@ -124,31 +124,38 @@ __device__ __forceinline__ void st_ff1(double* base, int m, FF v)
 }
 
 // FP64 <-> FP32 by the bits, on the integer pipes: a conversion that touches an
-// FP64 register issues at the FP64 rate.  widen: exact.  narrow: of a double
-// that is an FP32 number.  ff_split: the top 24 bits and the next 24 of a
-// double, as ff_of within 2^-48.  Zero and what lies outside FP32's normal
-// range take the conversion instructions.
+// FP64 register issues at the FP64 rate, and in a branch for rare values the
+// compiler would run it always and select.  widen: exact.  narrow: of a double
+// that is a normal FP32 number or zero.  ff_split: the top 24 bits and the next 24
+// of a double, as ff_of within 2^-48.  Below FP32's normal range narrow and
+// ff_split give zero, above it infinity; NaN stays NaN.
 __device__ __forceinline__ double widen(float f)
 {
-    const unsigned u = __float_as_uint(f), e = (u >> 23) & 0xffu;
-    if (e - 1u >= 254u) return (double)f;
-    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+    const bool sub = !(fabsf(f) >= 0x1p-126f);   // zero, subnormal or NaN
+    const unsigned u = __float_as_uint(sub ? f * 0x1p64f : f);
+    unsigned e = ((u >> 23) & 0xffu) + (sub ? 896u - 64u : 896u);
+    if (((u >> 23) & 0xffu) == 0xffu) e = 0x7ffu;
+    if ((u & 0x7fffffffu) == 0u) e = 0u;
+    return __hiloint2double((int)((u & 0x80000000u) | (e << 20) | ((u & 0x7fffffu) >> 3)), (int)(u << 29));
 }
 
 __device__ __forceinline__ float narrow(double d)
 {
     const unsigned h = (unsigned)__double2hiint(d), l = (unsigned)__double2loint(d), e = (h >> 20) & 0x7ffu;
-    if (e - 897u >= 254u) return (float)d;
-    return __uint_as_float((h & 0x80000000u) | (((h & 0x7fffffffu) - (896u << 20)) << 3) | (l >> 29));
+    unsigned v = (((h & 0x7fffffffu) - (896u << 20)) << 3) | (l >> 29);
+    if (e < 897u) v = 0u;
+    if (e > 1150u) v = e == 0x7ffu && ((h & 0xfffffu) | l) != 0u ? 0x7fffffffu : 0x7f800000u;
+    return __uint_as_float((h & 0x80000000u) | v);
 }
 
 __device__ __forceinline__ FF ff_split(double d)
 {
     const unsigned h = (unsigned)__double2hiint(d), l = (unsigned)__double2loint(d), e = (h >> 20) & 0x7ffu;
-    if (e - 960u >= 191u) return ff_of(d);   // |d| below 2^-63 or from 2^128
     const float hi = narrow(d);
-    const float lo = (float)(int)(l & 0x1fffffffu) * __uint_as_float((e - 948u) << 23 | (h & 0x80000000u));   // 2^(e - 1075)
-    return ff_renorm(hi, lo);
+    // the low 29 bits times 2^(e - 1075), the exponent in two steps that stay in range
+    const float lo = (float)(int)(l & 0x1fffffffu) * 0x1p-52f * __uint_as_float(((e - 896u) << 23 & 0x7f800000u) | (h & 0x80000000u));
+    const FF r = ff_renorm(hi, lo);
+    return e - 897u < 254u ? r : FF{hi, 0.f};
 }
 
 // a source vector's site as float-float: the Langevin sources are FP32 normals
