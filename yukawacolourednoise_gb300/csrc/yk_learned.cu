@@ -28,7 +28,7 @@
 
 #include <cuda_bf16.h>
 
-#include "yk_common.cuh"
+#include "yk_ff.cuh"
 #include "yk_kernels.h"
 
 namespace yk {
@@ -554,6 +554,15 @@ struct FusedLayers {
     int n;                      // layers in this launch (= the halo H)
 };
 
+constexpr int kPmMaxConv = 16;              // 2L of pcg_m_kernel
+constexpr size_t kPmMaxSmem = 200 * 1024;   // its shared memory
+__host__ __device__ inline size_t pm_smem(int R, int W, int H)
+{
+    // the two activation buffers, r' and sigma of the tile, the fragments
+    return 2 * sizeof(uint4) * (size_t)(R + 2 * H) * (W + 2 * H) + (sizeof(float4) + sizeof(float)) * (size_t)R * W +
+           sizeof(uint2) * 160 * (size_t)H;
+}
+
 __host__ __device__ inline int fused_region(int R, int W, int H) { return (R + 2 * H) * (W + 2 * H); }
 
 __global__ void __launch_bounds__(kNetThreads) net_conv_fused_kernel(const uint4* __restrict__ X,
@@ -720,6 +729,10 @@ struct LearnedNet {
     int restart = 0;
     PcgGraph* pcg = nullptr;          // its captured chunk of iterations
     bool pcg_no_graph = false;        // capture failed once (e.g. the legacy stream)
+    // an iteration in two launches (pcg_pq_kernel, pcg_m_kernel) on pm_R x pm_W tiles
+    // (pm_tiles 0: one launch per phase)
+    int pm_R = 0, pm_W = 0, pm_tiles = 0;
+    uint2* frag = nullptr;            // the layers' B fragments
     bool persistent = false;          // chunks of iterations as one cooperative launch (grid <= co-resident)
     unsigned* pbar = nullptr;         // its barrier counter and error word
 };
@@ -727,6 +740,7 @@ struct LearnedNet {
 namespace {
 
 int pcg_chunk_max_grid();
+void pcg_kernel_attributes();
 
 int cout_of(const LearnedNet* n, int l) { return l == n->layers - 1 ? kNetOut : kNetC; }
 
@@ -806,6 +820,7 @@ void net_destroy(LearnedNet* n)
         if (p) cudaFree(p);
     if (n->hpart) cudaFreeHost(n->hpart);
     if (n->pbar) cudaFree(n->pbar);
+    if (n->frag) cudaFree(n->frag);
     pcg_graph_destroy(n->pcg);
     for (uint4* h : n->h16)
         if (h) cudaFree(h);
@@ -816,9 +831,10 @@ int net_size(const LearnedNet* n) { return n->nw; }
 
 void net_tile(const LearnedNet* n, int* rows, int* cols, int* per_launch)
 {
-    *rows = n->tc_tuned ? n->tc_R : 0;
-    *cols = n->tc_tuned ? n->tc_W : 0;
-    *per_launch = n->tc_tuned ? n->tc_G : 0;
+    const bool pm = n->pm_tiles > 0;
+    *rows = pm ? n->pm_R : n->tc_tuned ? n->tc_R : 0;
+    *cols = pm ? n->pm_W : n->tc_tuned ? n->tc_W : 0;
+    *per_launch = pm ? 2 * n->layers : n->tc_tuned ? n->tc_G : 0;
 }
 
 bool net_tile_from_env(LearnedNet* n);
@@ -862,6 +878,7 @@ LearnedNet* net_create(int Nt, int Nx, int layers, cudaError_t* err)
     n->tc_R = kTcMaxR;
     cudaFuncSetAttribute((const void*)net_conv_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)kFusedMaxSmem);
+    pcg_kernel_attributes();
     while (n->tc_R > 2 && (int64_t)((Nt + n->tc_R - 1) / n->tc_R) * ((Nx + n->tc_W - 1) / n->tc_W) < 2 * n_sm)
         n->tc_R /= 2;
     cudaError_t e = alloc_f(&n->w, n->nw);
@@ -882,6 +899,7 @@ LearnedNet* net_create(int Nt, int Nx, int layers, cudaError_t* err)
     if (e == cudaSuccess) e = cudaMalloc(&n->h16[1], sizeof(uint4) * V);
     if (e == cudaSuccess) e = cudaMallocHost(&n->hpart, sizeof(double) * n->grid);
     if (e == cudaSuccess) e = cudaMalloc(&n->pbar, 2 * sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMalloc(&n->frag, sizeof(uint2) * 160 * 2 * (size_t)layers);
     if (e == cudaSuccess) n->hpart_cap = (size_t)n->grid;
     if (e == cudaSuccess) e = cudaMemset(n->m, 0, sizeof(float) * n->nw);
     if (e == cudaSuccess) e = cudaMemset(n->v, 0, sizeof(float) * n->nw);
@@ -890,7 +908,17 @@ LearnedNet* net_create(int Nt, int Nx, int layers, cudaError_t* err)
         net_destroy(n);
         n = nullptr;
     } else {
-        net_tile_from_env(n);
+        if (!net_tile_from_env(n) && !n->persistent && 2 * layers <= kPmMaxConv) {
+            // tiles of 8 x 64 sites; smaller while less than half the SMs would have one
+            int R = kTcMaxR, W = std::min(Nx, kTcMaxW);
+            auto tiles = [&] { return ((Nt + R - 1) / R) * ((Nx + W - 1) / W); };
+            while (tiles() < n_sm / 2 && (W > 16 || R > 2)) (W > 4 * R && W > 16 ? W : R) /= 2;
+            if (pm_smem(R, W, 2 * layers) <= kPmMaxSmem) {
+                n->pm_R = R;
+                n->pm_W = W;
+                n->pm_tiles = tiles();
+            }
+        }
     }
     *err = e;
     return n;
@@ -1717,10 +1745,382 @@ __global__ void __launch_bounds__(kNetThreads) pcg_dq_kernel(const float* __rest
     pcg_dq_body<true>(t, p, q, diag, part, Nt, Nx, rw);
 }
 
+// ---------------------------------------------------------------------------
+// An iteration in two launches (the default; YK_NET_TILE or YK_PCG_PERSISTENT
+// take the phases above one by one).  Only the two scalars need the whole
+// lattice, so everything between them is done on a tile that the block stages
+// with a halo as deep as the operators reach:
+//   pcg_pq_kernel  beta; p' = z + beta p on the tile and two sites around it,
+//                  D p' on one, q = D^dag D p' on the tile, <p', q>
+//   pcg_m_kernel   alpha; r' = r - alpha q on the tile and 2L sites around it, x,
+//                  the features, the network's 2L layers in shared memory, z = M r',
+//                  <r', z>, |r'|^2, <z, q>
+// r and p go to the other of two buffers, because a neighbour still reads the old
+// one.  The halo's work is done again in the neighbouring blocks (2.3 times the
+// tile's in the first of four layers of an 8 x 64 tile), but an iteration at
+// 512 x 512 with two layers went from 36 to 82 us in five to eight launches (by the
+// tile that was timed best) to 24 us.
+//
+// A layer's warp takes 16 sites of a row: ldmatrix brings the taps' 8 x 8 blocks
+// (a site's 8 channels are a row of 16 bytes) straight into the A fragments, five
+// loads and five products, against twenty 4-byte loads.
+// ---------------------------------------------------------------------------
+struct PmLayers {
+    const uint2* frag;   // B fragments of the tap pairs: [layer][5][32]
+    int n;               // 2L; the second half transposed
+};
+
+struct FragSource {
+    const float* w[kPmMaxConv];
+    int cout[kPmMaxConv];
+};
+
+// B fragments of every layer in the order they run (net_conv_bf_kernel's)
+__global__ void __launch_bounds__(160) net_frag_kernel(FragSource src, uint2* __restrict__ out)
+{
+    const int l = blockIdx.x, lane = threadIdx.x & 31, p = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+    const bool tr = l >= (int)gridDim.x / 2;
+    const int co = src.cout[l];
+    const float* Wl = src.w[l];
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int h = 0; h < 2; ++h) {
+        const int k = 2 * p + h;
+        if (k > 8) continue;
+        if (!tr) {
+            if (g < co) {
+                v[2 * h] = Wl[(k * kNetC + 2 * c) * co + g];
+                v[2 * h + 1] = Wl[(k * kNetC + 2 * c + 1) * co + g];
+            }
+        } else if (2 * c + 1 < co) {
+            v[2 * h] = Wl[(k * kNetC + g) * co + 2 * c];
+            v[2 * h + 1] = Wl[(k * kNetC + g) * co + 2 * c + 1];
+        }
+    }
+    out[(l * 5 + p) * 32 + lane] = make_uint2(pack_bf2(v[0], v[1]), pack_bf2(v[2], v[3]));
+}
+
+// Cells of a staged region of `cols` columns whose first cell is row tv0, column
+// x0 of the antiperiodically extended lattice: cell i is (row, col), lattice site n
+// with the extension's sign.
+struct Region {
+    int tv0, x0, cols, Nt, Nx;
+    unsigned magic;   // floor(2^32 / cols) + 1: i / cols for i < 2^16
+
+    __device__ __forceinline__ Region(int tv0_, int x0_, int cols_, int Nt_, int Nx_)
+        : tv0(tv0_), x0(x0_), cols(cols_), Nt(Nt_), Nx(Nx_), magic(0xffffffffu / (unsigned)cols_ + 1u)
+    {
+    }
+    __device__ __forceinline__ void cell(int i, int* row, int* col) const
+    {
+        *row = cols == 1 ? i : (int)__umulhi((unsigned)i, magic);
+        *col = i - *row * cols;
+    }
+    __device__ __forceinline__ int site(int row, int col, float* sign) const
+    {
+        int t = tv0 + row, x = x0 + col;
+        float s = 1.f;
+        while (t < 0) {
+            t += Nt;
+            s = -s;
+        }
+        while (t >= Nt) {
+            t -= Nt;
+            s = -s;
+        }
+        while (x < 0) x += Nx;
+        while (x >= Nx) x -= Nx;
+        *sign = s;
+        return t * Nx + x;
+    }
+};
+
+// Block sums of NV values, FP32 within a warp, float-float across the eight warps;
+// valid in thread 0.
+template <int NV>
+__device__ __forceinline__ void block_sum_ff(float (&v)[NV], float* red)
+{
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (lane == 0)
+#pragma unroll
+        for (int j = 0; j < NV; ++j) red[j * 8 + w] = v[j];
+    __syncthreads();
+    if (w == 0)
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            FF t = {lane < 8 ? red[j * 8 + lane] : 0.f, 0.f};
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) t = ff_add(t, ff_shfl_xor(t, o));
+            v[j] = t.hi + t.lo;
+        }
+}
+
+// The totals of two arrays of nb per-block partials in every thread, in a fixed
+// order (the same bits in every block).
+__device__ __forceinline__ float2 tile_totals(const float* a, const float* b, int nb, float2* wsum)
+{
+    float sa = 0.f, sb = 0.f;
+    for (int i = threadIdx.x; i < nb; i += kNetThreads) {
+        sa += __ldcg(a + i);
+        sb += __ldcg(b + i);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        sa += __shfl_xor_sync(0xffffffffu, sa, o);
+        sb += __shfl_xor_sync(0xffffffffu, sb, o);
+    }
+    if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = make_float2(sa, sb);
+    __syncthreads();
+    float2 t = wsum[threadIdx.x & 7];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
+        t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
+    }
+    return t;
+}
+
+__device__ __forceinline__ float dot4(float4 a, float4 b) { return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, a.w * b.w))); }
+
+struct PcgTile {
+    int Nt, Nx, R, W;
+};
+
+__global__ void __launch_bounds__(kNetThreads, 4) pcg_m_kernel(const float4* __restrict__ r, float4* __restrict__ r_out,
+                                                            float4* __restrict__ x, const float4* __restrict__ p,
+                                                            const float4* __restrict__ q, float4* __restrict__ z,
+                                                            const float* __restrict__ sigma,
+                                                            const float* __restrict__ part_rz,
+                                                            const float* __restrict__ part_pq,
+                                                            float* __restrict__ part, PmLayers L, PcgTile T, float skip,
+                                                            int first)
+{
+    extern __shared__ __align__(16) uint4 pm_raw[];
+    __shared__ float red[24];
+    __shared__ float2 wsum[8];
+    const int H = L.n, R = T.R, W = T.W, Nt = T.Nt, Nx = T.Nx, nb = gridDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint4* in = pm_raw;
+    uint4* out = in + (R + 2 * H) * (W + 2 * H);
+    float4* const rs = reinterpret_cast<float4*>(out + (R + 2 * H) * (W + 2 * H));
+    uint2* const frag = reinterpret_cast<uint2*>(rs + R * W);
+    float* const sg = reinterpret_cast<float*>(frag + 160 * H);
+    for (int i = threadIdx.x; i < 160 * H; i += kNetThreads) frag[i] = L.frag[i];   // constant during a solve
+    const int tiles_x = (Nx + W - 1) / W;
+    const int t0 = (blockIdx.x / tiles_x) * R, x0 = (blockIdx.x % tiles_x) * W;
+    const int Rt = min(R, Nt - t0), Wt = min(W, Nx - x0), SC = Wt + 2 * H, cells = (Rt + 2 * H) * SC;
+    const Region G(t0 - H, x0 - H, SC, Nt, Nx);
+    pdl_wait();
+    float a = 0.f;
+    constexpr int kB = 4;   // sites a thread has on their way; the first while the totals come
+    for (int base = threadIdx.x; base - (int)threadIdx.x < cells; base += kB * kNetThreads) {
+        float4 rv[kB], qv[kB];
+        float sv[kB], sign[kB];
+        int row[kB], col[kB], n[kB];
+#pragma unroll
+        for (int e = 0; e < kB; ++e) {
+            const int i = base + e * kNetThreads;
+            n[e] = -1;
+            if (i < cells) {
+                G.cell(i, &row[e], &col[e]);
+                n[e] = G.site(row[e], col[e], &sign[e]);
+                rv[e] = r[n[e]];
+                if (!first) qv[e] = q[n[e]];
+                sv[e] = sigma[n[e]];
+            }
+        }
+        if (!first && base == (int)threadIdx.x) {
+            const float2 t = tile_totals(part_rz, part_pq, nb, wsum);
+            a = t.y != 0.f ? t.x / t.y : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < kB; ++e) {
+            if (n[e] < 0) continue;
+            float4 v = rv[e];
+            if (!first)
+                v = make_float4(fmaf(-a, qv[e].x, v.x), fmaf(-a, qv[e].y, v.y), fmaf(-a, qv[e].z, v.z),
+                                fmaf(-a, qv[e].w, v.w));
+            const int lr = row[e] - H, lc = col[e] - H;
+            if ((unsigned)lr < (unsigned)Rt && (unsigned)lc < (unsigned)Wt) {
+                rs[lr * Wt + lc] = v;
+                sg[lr * Wt + lc] = sv[e];
+                if (!first) r_out[n[e]] = v;
+            }
+            if (H > 0)
+                in[base + e * kNetThreads] =
+                    features_bf(make_float4(sign[e] * v.x, sign[e] * v.y, sign[e] * v.z, sign[e] * v.w), sv[e]);
+        }
+    }
+    __syncthreads();
+    pdl_trigger();
+    // the layers: layer j's region is the tile widened by H - 1 - j
+    const int ms = (lane & 7) + ((lane >> 3) & 1) * 8;   // the lane's site of 16 in the ldmatrix, its tap of two
+    const int mt = lane >> 4;
+    for (int j = 0; j < H; ++j) {
+        const int hout = H - 1 - j, SWi = Wt + 2 * (hout + 1), RO = Rt + 2 * hout, WO = Wt + 2 * hout;
+        const bool tr = j >= H / 2;
+        uint2 b[5];
+        int off[5];   // bytes
+#pragma unroll
+        for (int pr = 0; pr < 5; ++pr) {
+            b[pr] = frag[(j * 5 + pr) * 32 + lane];
+            int k = 2 * pr + (pr < 4 ? mt : 0);   // the pair's missing last tap has zero weights
+            if (tr) k = 8 - k;
+            off[pr] = 16 * ((k / 3) * SWi + k % 3);
+        }
+        const unsigned ia = (unsigned)__cvta_generic_to_shared(in);
+        const unsigned oa = (unsigned)__cvta_generic_to_shared(out) + 16u * (unsigned)(lane >> 2) + 4u * (unsigned)(lane & 3);
+        // the units of 16 sites, down one strip of columns after another, in equal
+        // shares of the warps
+        const int strips = (WO + 15) / 16, total = strips * RO;
+        const unsigned dat = 16u * (unsigned)SWi, dto = 16u * (unsigned)WO;
+        int u = total * warp / (kNetThreads / 32);
+        const int u1 = total * (warp + 1) / (kNetThreads / 32);
+        for (int strip = u / RO, row = u - strip * RO; u < u1; ++strip, row = 0) {
+            const int col0 = strip * 16, c = col0 + (lane >> 2), rows = min(RO - row, u1 - u);
+            const bool st0 = c < WO, st1 = c + 8 < WO;
+            unsigned at = ia + 16u * (unsigned)(row * SWi + min(col0 + ms, WO - 1));
+            unsigned to = oa + 16u * (unsigned)(row * WO + col0);
+            u += rows;
+#pragma unroll 2
+            for (int k = 0; k < rows; ++k, at += dat, to += dto) {
+                float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int pr = 0; pr < 5; ++pr) {
+                    uint32_t m[4];
+                    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                                 : "=r"(m[0]), "=r"(m[1]), "=r"(m[2]), "=r"(m[3])
+                                 : "r"(at + off[pr])
+                                 : "memory");
+                    mma_bf16(acc, m, b[pr].x, b[pr].y);
+                }
+                if (st0) asm volatile("st.shared.b32 [%0], %1;" ::"r"(to), "r"(pack_bf2(acc[0], acc[1])) : "memory");
+                if (st1) asm volatile("st.shared.b32 [%0], %1;" ::"r"(to + 128u), "r"(pack_bf2(acc[2], acc[3])) : "memory");
+            }
+        }
+        __syncthreads();
+        uint4* const tmp = in;
+        in = out;
+        out = tmp;
+    }
+    float acc[3] = {0.f, 0.f, 0.f};
+    const Region O(t0, x0, Wt, Nt, Nx);
+    for (int i = threadIdx.x; i < Rt * Wt; i += kNetThreads) {
+        int lr, lc;
+        O.cell(i, &lr, &lc);
+        const int n = (t0 + lr) * Nx + x0 + lc;
+        const float4 rv = rs[i];
+        const float4 o = H > 0 ? featT_bf(in[i], sg[i], rv, skip) : rv;
+        z[n] = o;
+        acc[0] += dot4(rv, o);
+        acc[1] += dot4(rv, rv);
+        if (!first) {
+            const float4 pv = p[n], xv = x[n];
+            acc[2] += dot4(o, q[n]);
+            x[n] = make_float4(fmaf(a, pv.x, xv.x), fmaf(a, pv.y, xv.y), fmaf(a, pv.z, xv.z), fmaf(a, pv.w, xv.w));
+        }
+    }
+    block_sum_ff<3>(acc, red);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = acc[0];
+        part[nb + blockIdx.x] = acc[1];
+        part[2 * nb + blockIdx.x] = acc[2];
+    }
+}
+
+__host__ __device__ inline size_t pq_smem(int R, int W)
+{
+    return sizeof(float4) * ((size_t)(R + 4) * (W + 4) + (size_t)(R + 2) * (W + 2));
+}
+
+__global__ void __launch_bounds__(kNetThreads, 4) pcg_pq_kernel(const float4* __restrict__ z, const float4* __restrict__ p,
+                                                             float4* __restrict__ p_new, float4* __restrict__ q,
+                                                             const float* __restrict__ diag,
+                                                             const float* __restrict__ part_zq, float* __restrict__ part_pq,
+                                                             const float* __restrict__ part_pq_old, PcgTile T, float rw)
+{
+    extern __shared__ __align__(16) float4 pq_raw[];
+    __shared__ float red[8];
+    __shared__ float2 wsum[8];
+    const int R = T.R, W = T.W, Nt = T.Nt, Nx = T.Nx, nb = gridDim.x;
+    const int tiles_x = (Nx + W - 1) / W;
+    const int t0 = (blockIdx.x / tiles_x) * R, x0 = (blockIdx.x % tiles_x) * W;
+    const int Rt = min(R, Nt - t0), Wt = min(W, Nx - x0), SP = Wt + 4, ST = Wt + 2;
+    float4* const ps = pq_raw;
+    float4* const ts = ps + (R + 4) * (W + 4);
+    const Region G(t0 - 2, x0 - 2, SP, Nt, Nx), M(t0 - 1, x0 - 1, ST, Nt, Nx), O(t0, x0, Wt, Nt, Nx);
+    const int cells = (Rt + 4) * SP;
+    pdl_wait();
+    float b = 0.f;
+    constexpr int kB = 4;
+    for (int base = threadIdx.x; base - (int)threadIdx.x < cells; base += kB * kNetThreads) {
+        float4 zv[kB], pv[kB];
+        float sign[kB];
+        int row[kB], col[kB], n[kB];
+#pragma unroll
+        for (int e = 0; e < kB; ++e) {
+            const int i = base + e * kNetThreads;
+            n[e] = -1;
+            if (i < cells) {
+                G.cell(i, &row[e], &col[e]);
+                n[e] = G.site(row[e], col[e], &sign[e]);
+                zv[e] = z[n[e]];
+                pv[e] = p[n[e]];
+            }
+        }
+        if (base == (int)threadIdx.x) {
+            const float2 t = tile_totals(part_zq, part_pq_old, nb, wsum);
+            b = t.y != 0.f ? -t.x / t.y : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < kB; ++e) {
+            if (n[e] < 0) continue;
+            const float4 v = make_float4(fmaf(b, pv[e].x, zv[e].x), fmaf(b, pv[e].y, zv[e].y), fmaf(b, pv[e].z, zv[e].z),
+                                         fmaf(b, pv[e].w, zv[e].w));
+            if ((unsigned)(row[e] - 2) < (unsigned)Rt && (unsigned)(col[e] - 2) < (unsigned)Wt) p_new[n[e]] = v;
+            ps[base + e * kNetThreads] = make_float4(sign[e] * v.x, sign[e] * v.y, sign[e] * v.z, sign[e] * v.w);
+        }
+    }
+    __syncthreads();
+    pdl_trigger();
+    auto at = [](const float4* s) {
+        const float4 v = *s;
+        return Site<float, 1>{{v.x, v.y, v.z, v.w}};
+    };
+    for (int i = threadIdx.x; i < (Rt + 2) * ST; i += kNetThreads) {
+        int lr, lc;
+        float sign;
+        M.cell(i, &lr, &lc);
+        const float4* c = ps + (lr + 1) * SP + lc + 1;
+        const Site<float, 1> o = dirac_combine<float, 1, false>(at(c), at(c + SP), at(c - SP), at(c + 1), at(c - 1),
+                                                                diag[M.site(lr, lc, &sign)], rw, 1.f, 1.f);
+        ts[i] = make_float4(o.v[0], o.v[1], o.v[2], o.v[3]);
+    }
+    __syncthreads();
+    float acc[1] = {0.f};
+    for (int i = threadIdx.x; i < Rt * Wt; i += kNetThreads) {
+        int lr, lc;
+        O.cell(i, &lr, &lc);
+        const int n = (t0 + lr) * Nx + x0 + lc;
+        const float4* c = ts + (lr + 1) * ST + lc + 1;
+        const Site<float, 1> o = dirac_combine<float, 1, true>(at(c), at(c + ST), at(c - ST), at(c + 1), at(c - 1), diag[n],
+                                                               rw, 1.f, 1.f);
+        const float4 qv = make_float4(o.v[0], o.v[1], o.v[2], o.v[3]);
+        q[n] = qv;
+        acc[0] += dot4(ps[(lr + 2) * SP + lc + 2], qv);
+    }
+    block_sum_ff<1>(acc, red);
+    if (threadIdx.x == 0) part_pq[blockIdx.x] = acc[0];
+}
+
 struct PcgBufs {
-    float *r, *x, *z, *p[2], *q, *tmp;
+    float *r, *x, *z, *p[2], *q, *tmp;   // tmp: D p', or (two launches) the other r
     float* part_z;    // 3 x grid FP32 partials of the z kernel: <r, z>, <r, r>, <z, q>
     float* part_pq;   // grid FP32 partials of <p, q>
+    float* part[2];   // two launches, by parity: the same four, each a tile's
 };
 
 // ---------------------------------------------------------------------------
@@ -1813,6 +2213,12 @@ __global__ void __launch_bounds__(kNetThreads) pcg_chunk_kernel(PcgChunk P)
     }
 }
 
+void pcg_kernel_attributes()
+{
+    cudaFuncSetAttribute((const void*)pcg_m_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPmMaxSmem);
+    cudaFuncSetAttribute((const void*)pcg_pq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPmMaxSmem);
+}
+
 // Blocks of pcg_chunk_kernel that fit on the device at once (0: none).
 int pcg_chunk_max_grid()
 {
@@ -1845,6 +2251,19 @@ void pcg_precond(LearnedNet* n, bool use_net, const DiracArgs& d, const PcgBufs&
                (const float*)(first ? nullptr : b.q), b.part_z, V);
 }
 
+// z = M r, x and r' (two launches an iteration; first: z = M r of the given r)
+void pcg_m(LearnedNet* n, bool use_net, const DiracArgs& d, const PcgBufs& b, bool first, int parity, cudaStream_t s)
+{
+    const PcgTile T = {n->Nt, n->Nx, n->pm_R, n->pm_W};
+    const int H = use_net ? 2 * n->layers : 0, nb = n->pm_tiles, to = first ? parity : parity ^ 1;
+    const float* rr = parity ? b.tmp : b.r;
+    launch_pdl(pcg_m_kernel, nb, pm_smem(T.R, T.W, H), s, reinterpret_cast<const float4*>(rr),
+               reinterpret_cast<float4*>(parity ? b.r : b.tmp), reinterpret_cast<float4*>(b.x),
+               reinterpret_cast<const float4*>(b.p[to]), reinterpret_cast<const float4*>(b.q),
+               reinterpret_cast<float4*>(b.z), (const float*)n->sig32, (const float*)b.part[parity],
+               (const float*)(b.part[to] + 3 * nb), b.part[to], PmLayers{n->frag, H}, T, n->skip, first ? 1 : 0);
+}
+
 // `count` iterations from the direction buffer `parity`: p' = z + beta p and
 // t = D p', q = D^dag t with alpha, x and r (and the features of r),
 // z = M r with beta.  Returns the parity after them.
@@ -1853,6 +2272,20 @@ int pcg_iterations(LearnedNet* n, bool use_net, const DiracArgs& d, const PcgBuf
 {
     const int V = n->V, nb = n->grid;
     const float rw = (float)d.r;
+    if (n->pm_tiles) {
+        const PcgTile T = {n->Nt, n->Nx, n->pm_R, n->pm_W};
+        const int nt = n->pm_tiles;
+        for (int it = 0; it < count; ++it, parity ^= 1) {
+            const int to = parity ^ 1;
+            launch_pdl(pcg_pq_kernel, nt, pq_smem(T.R, T.W), s, reinterpret_cast<const float4*>(b.z),
+                       reinterpret_cast<const float4*>(b.p[parity]), reinterpret_cast<float4*>(b.p[to]),
+                       reinterpret_cast<float4*>(b.q), (const float*)n->diag32,
+                       (const float*)(b.part[parity] + 2 * nt), b.part[to] + 3 * nt,
+                       (const float*)(b.part[parity] + 3 * nt), T, rw);
+            pcg_m(n, use_net, d, b, false, parity, s);
+        }
+        return parity;
+    }
     if (n->persistent && count > 0 && (!use_net || n->tc_G == 1)) {
         PcgChunk P = {};
         P.z = b.z;
@@ -1941,32 +2374,45 @@ static cudaError_t pcg_solve_once(LearnedNet* n, bool use_net, const double* sig
     const int V4 = 4 * n->V;
     const DiracArgs d = {sigma, n->Nt, n->Nx, m0, g, r};
     cudaError_t e = ensure_scratch(n, 2);   // Zs, Ws: two 4V float vectors each
-    if (e == cudaSuccess) e = ensure_parts(n, 4);
+    const int nt = n->pm_tiles;
+    if (e == cudaSuccess) e = ensure_parts(n, std::max(4, (4 * nt + n->grid - 1) / n->grid));
     if (e != cudaSuccess) return e;
     double* Ax = n->d1;
     double* r64 = n->d2;
     float* fpart = reinterpret_cast<float*>(n->dpart);   // 4 x grid floats in the partials' space
     const PcgBufs B = {n->f0, n->f1, n->f2, {n->Zs, n->Zs + (size_t)V4}, n->Ws, n->f3, fpart,
-                       fpart + 3 * (size_t)n->grid};
+                       fpart + 3 * (size_t)n->grid, {fpart, fpart + 4 * (size_t)nt}};
+    int parity = 0;
     // |r|^2 of the inner solve from the z kernel's partials (host sum)
     auto inner_rr = [&](double* out) -> cudaError_t {
+        const int np = nt ? nt : n->grid;
         float* hf = reinterpret_cast<float*>(n->hpart);
-        unsigned* hbad = reinterpret_cast<unsigned*>(hf + n->grid);   // the persistent chunk's error word
+        unsigned* hbad = reinterpret_cast<unsigned*>(hf + np);   // the persistent chunk's error word
         *hbad = 0u;
-        cudaError_t ce = cudaMemcpyAsync(hf, B.part_z + n->grid, sizeof(float) * n->grid, cudaMemcpyDeviceToHost, s);
+        cudaError_t ce = cudaMemcpyAsync(hf, (nt ? B.part[parity] : B.part_z) + np, sizeof(float) * np,
+                                         cudaMemcpyDeviceToHost, s);
         if (ce == cudaSuccess && n->persistent)
             ce = cudaMemcpyAsync(hbad, n->pbar + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(s);
         if (ce == cudaSuccess && *hbad) ce = cudaErrorLaunchTimeout;   // a barrier wait gave up
         double t = 0.0;
-        for (int i = 0; i < n->grid; ++i) t += hf[i];
+        for (int i = 0; i < np; ++i) t += hf[i];
         *out = t;
         return ce;
     };
     f_of_d_kernel<<<n->grid, kNetThreads, 0, s>>>(sigma, n->sig32, n->V);
     diag_f_kernel<<<n->grid, kNetThreads, 0, s>>>(sigma, n->diag32, m0, g, r, n->V);
     const int nb = n->grid;
-    if (use_net && !n->tc_tuned) {
+    if (use_net && nt) {
+        FragSource src = {};
+        const int L = n->layers;
+        for (int q = 0; q < 2 * L; ++q) {
+            const int l = q < L ? q : 2 * L - 1 - q;   // N's layers, then N^T's in reverse
+            src.w[q] = n->w + n->woff[l];
+            src.cout[q] = cout_of(n, l);
+        }
+        net_frag_kernel<<<2 * L, 160, 0, s>>>(src, n->frag);
+    } else if (use_net && !n->tc_tuned) {
         e = net_tune_tile(n, s);
         if (e != cudaSuccess) return e;
         if (n->pcg) {   // captured with the previous tile
@@ -2021,10 +2467,14 @@ static cudaError_t pcg_solve_once(LearnedNet* n, bool use_net, const double* sig
         e = cudaMemsetAsync(B.x, 0, sizeof(float) * V4, s);
         if (e == cudaSuccess) e = cudaMemsetAsync(B.p[0], 0, sizeof(float) * V4, s);
         // zero <p, q> partials: the first direction takes beta = 0, p' = z
-        if (e == cudaSuccess) e = cudaMemsetAsync(B.part_pq, 0, sizeof(float) * nb, s);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(nt ? B.part[0] + 3 * nt : B.part_pq, 0, sizeof(float) * (nt ? nt : nb), s);
         if (e != cudaSuccess) break;
-        pcg_precond(n, use_net, d, B, true, s);   // z = M r
-        int parity = 0;
+        parity = 0;
+        if (nt)
+            pcg_m(n, use_net, d, B, true, 0, s);   // z = M r
+        else
+            pcg_precond(n, use_net, d, B, true, s);
         double rr0 = 0.0;
         e = inner_rr(&rr0);
         double rrc = rr0;
