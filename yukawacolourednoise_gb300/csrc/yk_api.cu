@@ -70,6 +70,8 @@ struct Workspace {
     double* corr = nullptr;     // Nt
 };
 
+struct PlaneWs;
+
 struct Chain {
     yk_params p;
     yk_action a;
@@ -84,6 +86,7 @@ struct Chain {
     uint8_t* keep;
     double2 *tw_t, *tw_x;
     Workspace ws;
+    PlaneWs* planes = nullptr;   // of mixed solves of complex sources (launch_plane_solve)
     LearnedNet* net = nullptr;   // the learned preconditioner (yk_net_setup)
     LearnedNet* pcg_ws = nullptr;   // solver buffers of identity-preconditioned solves without a network
     // pion extension (params.pions): the fields pi_1..3 (3V), their coloured
@@ -637,12 +640,158 @@ int ensure_ws(yk_ctx* ctx, int c, int R)
     return YK_OK;
 }
 
+// The two real plane systems of chain c for launch_plane_solve (one allocation, on
+// the first such solve).
+struct PlaneWs {
+    void* mem = nullptr;
+    SysDev *sys, *eo;
+    int2* tiles;
+    CGState* st;      // four: two solves of two planes
+    Partial* partial;
+    double *norm, *resid, *stop2, *tmp;
+};
+
+int ensure_planes(yk_ctx* ctx, int c)
+{
+    Chain& C = ctx->ch[c];
+    if (C.planes) return YK_OK;
+    const size_t V = C.V, Ve = V / 2, nt = ntiles_of(C.V);
+    Arena ar;
+    const size_t o_sys = ar.reserve(4 * sizeof(SysDev)), o_tiles = ar.reserve(2 * nt * sizeof(int2));
+    const size_t o_st = ar.reserve(4 * sizeof(CGState)), o_part = ar.reserve(2 * nt * sizeof(Partial));
+    const size_t o_norm = ar.reserve(plane_norm_doubles() * 8), o_resid = ar.reserve(plane_norm_doubles() * 8);
+    const size_t o_stop = ar.reserve(5 * 8), o_tmp = ar.reserve(2 * 64 * V);
+    size_t o_b[2], o_x[2], o_t[2], o_dinv[2], o_de[2], o_p[2];
+    for (int k = 0; k < 2; ++k) {
+        o_b[k] = ar.reserve(32 * V);
+        o_x[k] = ar.reserve(32 * V);
+        o_t[k] = ar.reserve(32 * Ve);
+        o_dinv[k] = ar.reserve(8 * Ve);
+        o_de[k] = ar.reserve(8 * Ve);
+        o_p[k] = ar.reserve(16 * Ve);
+    }
+    std::unique_ptr<PlaneWs> w(new PlaneWs());
+    if (cudaMalloc(&w->mem, ar.used) != cudaSuccess) {
+        cudaGetLastError();
+        set_error("plane workspace allocation of %zu bytes failed", ar.used);
+        return YK_ENOMEM;
+    }
+    ar.base = (char*)w->mem;
+    w->sys = ar.at<SysDev>(o_sys);
+    w->eo = w->sys + 2;
+    w->tiles = ar.at<int2>(o_tiles);
+    w->st = ar.at<CGState>(o_st);
+    w->partial = ar.at<Partial>(o_part);
+    w->norm = ar.at<double>(o_norm);
+    w->resid = ar.at<double>(o_resid);
+    w->stop2 = ar.at<double>(o_stop);
+    w->tmp = ar.at<double>(o_tmp);
+    std::vector<SysDev> h(4, SysDev());
+    std::vector<int2> tiles(2 * nt, make_int2(0, 0));
+    for (int k = 0; k < 2; ++k) {
+        SysDev& S = h[k];
+        S.chain = c;
+        S.rhs = k;
+        S.Nt = C.Nt;
+        S.Nx = C.Nx;
+        S.V = C.V;
+        S.tile0 = (int)(k * nt);
+        S.ntiles = (int)nt;
+        S.m0 = C.a.m0;
+        S.g = C.a.g;
+        S.r = C.a.r;
+        S.sigma = C.phi;
+        S.b = ar.at<double>(o_b[k]);
+        S.x = ar.at<double>(o_x[k]);
+        S.t64 = ar.at<double>(o_t[k]);
+        S.p32[0] = S.p32[1] = ar.at<float>(o_p[k]);
+        SysDev& E = h[2 + k];
+        E = S;
+        E.Nx = C.Nx / 2;
+        E.V = (int)Ve;
+        E.ntiles = ntiles_of((int)Ve);
+        E.dinv = ar.at<double>(o_dinv[k]);
+        E.v32 = ar.at<float>(o_de[k]);
+        for (int t = 0; t < E.ntiles; ++t) tiles[E.tile0 + t] = make_int2(k, t * kTile);
+    }
+    cudaError_t e = cudaMemcpyAsync(w->sys, h.data(), sizeof(SysDev) * 4, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(w->tiles, tiles.data(), sizeof(int2) * tiles.size(), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) {
+        cudaFree(w->mem);
+        YK_CK(e);
+    }
+    C.planes = w.release();
+    return YK_OK;
+}
+
+// A mixed solve of one complex source on a lattice that cg_eoc_kernel takes.
+// *done false: it did not reach the target on the FP64 residual (or within
+// max_iter), and the caller solves otherwise.
+int plane_solve(yk_ctx* ctx, int c, const EocForm& form, int mtype, double tol, int tol_mode, int max_iter,
+                yk_solve_stats* stats, bool* done)
+{
+    Chain& C = ctx->ch[c];
+    *done = false;
+    if (int rc = ensure_planes(ctx, c)) return rc;
+    const PlaneWs& w = *C.planes;
+    const SysDev& S = C.ws.h_sys[0];
+    CGArgs a = base_args(ctx);
+    a.sys = w.sys;
+    a.sys_eo = w.eo;
+    a.sys_first = 0;
+    a.sys_count = 2;
+    a.eo_tiles = w.tiles;
+    a.tile_begin = 0;
+    a.tile_end = 2 * ntiles_of(C.V);
+    a.st = w.st;
+    a.partial = w.partial;
+    a.mtype = mtype;
+    a.tol = tol;
+    a.tol_mode = tol_mode;
+    a.max_iter = max_iter;
+    YK_CK(launch_plane_solve(a, form, S.b, S.x, C.phi, C.Nt, C.Nx, C.a.m0, C.a.g, C.a.r, w.norm, w.resid, w.stop2, w.tmp,
+                             ctx->stream));
+    CGState st[4];
+    const size_t half = plane_norm_doubles() / 2;
+    std::vector<double> n(2 * half);
+    YK_CK(cudaMemcpyAsync(st, w.st, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
+    YK_CK(cudaMemcpyAsync(n.data(), w.norm, 8 * half, cudaMemcpyDeviceToHost, ctx->stream));
+    YK_CK(cudaMemcpyAsync(n.data() + half, w.resid, 8 * half, cudaMemcpyDeviceToHost, ctx->stream));
+    if (int rc = status_of_err(ctx)) return rc;
+    yk_solve_stats s = {};
+    for (size_t i = 0; i < half; ++i) {
+        s.rr0 += n[i];
+        s.rr += n[half + i];
+    }
+    bool ok = true;
+    for (int k = 0; k < 4; k += 2) {   // a solve's planes run side by side
+        s.iterations += std::max(st[k].iters, st[k + 1].iters);
+        s.reliable_updates += std::max(st[k].n_ru, st[k + 1].n_ru);
+        ok = ok && st[k].converged && st[k + 1].converged;
+    }
+    s.converged = 1;
+    const double stop2 = tol_mode == YK_TOL_ABS ? tol * tol : tol * tol * s.rr0;
+    *done = ok && !(s.rr > stop2) && s.rr == s.rr && s.iterations <= max_iter;
+    if (*done && stats) *stats = s;
+    return YK_OK;
+}
+
 // Solves the first `count` systems of chain c's complex workspace.
 int ws_solve(yk_ctx* ctx, int c, int count, int mtype, double tol, int tol_mode, int max_iter, int precision,
              yk_solve_stats* stats)
 {
     Chain& C = ctx->ch[c];
     Workspace& w = C.ws;
+    EocForm form;
+    const char* eo = getenv("YK_CG_EO");
+    if (count == 1 && precision == YK_MIXED && !C.pions && C.Nt % 2 == 0 && C.Nx % 2 == 0 && C.Nx >= 4 &&
+        !(eo && eo[0] == '0') && cg_eoc_form(C.Nt, C.Nx / 2, C.a.r, kEocSpread, &form)) {
+        bool done = false;
+        if (int rc = plane_solve(ctx, c, form, mtype, tol, tol_mode, max_iter, stats, &done)) return rc;
+        if (done) return YK_OK;
+    }
     YK_CK(cudaMemcpyAsync(w.d_sys, w.h_sys.data(), sizeof(SysDev) * count, cudaMemcpyHostToDevice, ctx->stream));
     CGArgs a = base_args(ctx);
     a.sys = w.d_sys;
@@ -1228,7 +1377,7 @@ int yk_ctx_create(const yk_params* params, int n_chains, yk_ctx** out)
     cg_max_grid(2, true);
     if (mixed) cg_halo_init();
     cg_small_init();
-    if (mixed) cg_eoc_init();
+    cg_eoc_init();
     noise_init_attributes();
     {
         // opt-in while its FP64 reliable updates run on 16 SMs only
@@ -1572,6 +1721,10 @@ int yk_ctx_destroy(yk_ctx* ctx)
     for (auto e : ctx->pool) cudaEventDestroy(e);
     for (auto& C : ctx->ch) {
         if (C.ws.mem) cudaFree(C.ws.mem);
+        if (C.planes) {
+            cudaFree(C.planes->mem);
+            delete C.planes;
+        }
         if (C.series) cudaFree(C.series);
         net_destroy(C.net);
         net_destroy(C.pcg_ws);

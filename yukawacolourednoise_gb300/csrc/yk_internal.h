@@ -149,6 +149,8 @@ struct CGArgs {
     // relative to |eta|^2, tile partial slot 5 of round 0
     const SysDev* sys_full;
     int eo;
+    // cg_eoc_kernel: each system's target on |r|^2 by its rhs (null: from tol)
+    const double* stop2;
 };
 
 // The one lattice of all systems of a solve, for cg_small_kernel (Nt 0: they differ).

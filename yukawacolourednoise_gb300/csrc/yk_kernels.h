@@ -38,6 +38,11 @@ bool cg_eoc_form(int Nt, int Nh, double r, int spread, EocForm* f);
 cudaError_t launch_cg_eoc(const CGArgs& a, const EocForm& f, const int* order, int count, cudaStream_t stream);
 cudaError_t launch_eoc_prepare(const CGArgs& a, bool r1, bool other, int max_nh, cudaStream_t stream);
 void cg_eoc_init();
+// A x = b for a complex source by two such solves of its planes (yk_cg_eoc.cu).
+size_t plane_norm_doubles();
+cudaError_t launch_plane_solve(const CGArgs& a, const EocForm& f, const double* b, double* x, const double* sigma, int Nt,
+                               int Nx, double m0, double g, double r, double* norm, double* resid, double* stop2,
+                               double* tmp, cudaStream_t stream);
 // Work-balanced block ranges (CGArgs::balance) for the next solve of the
 // systems of `a`, from their iteration counts in the solve just finished;
 // grid: the grid of that solve's launch.  No-op for a single system.
