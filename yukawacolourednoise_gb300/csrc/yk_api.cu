@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <new>
 #include <string>
@@ -778,15 +779,16 @@ int plane_solve(yk_ctx* ctx, int c, const EocForm& form, int mtype, double tol, 
     return YK_OK;
 }
 
-// Solves the first `count` systems of chain c's complex workspace.
+// Solves the first `count` systems of chain c's complex workspace.  beside(), when
+// given, is called once the solve has been launched, before it is waited for.
 int ws_solve(yk_ctx* ctx, int c, int count, int mtype, double tol, int tol_mode, int max_iter, int precision,
-             yk_solve_stats* stats)
+             yk_solve_stats* stats, const std::function<int()>& beside = nullptr)
 {
     Chain& C = ctx->ch[c];
     Workspace& w = C.ws;
     EocForm form;
     const char* eo = getenv("YK_CG_EO");
-    if (count == 1 && precision == YK_MIXED && !C.pions && C.Nt % 2 == 0 && C.Nx % 2 == 0 && C.Nx >= 4 &&
+    if (count == 1 && precision == YK_MIXED && !C.pions && !beside && C.Nt % 2 == 0 && C.Nx % 2 == 0 && C.Nx >= 4 &&
         !(eo && eo[0] == '0') && cg_eoc_form(C.Nt, C.Nx / 2, C.a.r, kEocSpread, &form)) {
         bool done = false;
         if (int rc = plane_solve(ctx, c, form, mtype, tol, tol_mode, max_iter, stats, &done)) return rc;
@@ -809,6 +811,8 @@ int ws_solve(yk_ctx* ctx, int c, int count, int mtype, double tol, int tol_mode,
     a.tol_mode = tol_mode;
     a.max_iter = max_iter;
     YK_CK(launch_cg(a, 2, precision == YK_MIXED, ctx->stream, nullptr, nullptr, {C.Nt, C.Nx, C.pions ? 1 : 0}));
+    if (beside)
+        if (int rc = beside()) return rc;
     std::vector<CGState> st(count);
     YK_CK(cudaMemcpyAsync(st.data(), w.d_state, sizeof(CGState) * count, cudaMemcpyDeviceToHost, ctx->stream));
     int rc = status_of_err(ctx);
@@ -1284,7 +1288,8 @@ void eo_args(const yk_ctx* ctx, CGArgs& a)
 // The complex systems of a pion chain: sources eta (device, n_rhs x 8V) or,
 // when null, Philox stream `kind` at the chain's current step; solved with
 // the pion operator on the chain's workspace.
-int pion_solve(yk_ctx* ctx, int c, int kind, const double* eta, int precision, yk_solve_stats* stats)
+int pion_solve(yk_ctx* ctx, int c, int kind, const double* eta, int precision, yk_solve_stats* stats,
+               const std::function<int()>& beside = nullptr)
 {
     Chain& C = ctx->ch[c];
     const int R = C.n_rhs_pion;
@@ -1299,7 +1304,7 @@ int pion_solve(yk_ctx* ctx, int c, int kind, const double* eta, int precision, y
         eta = C.peta;
     }
     for (int j = 0; j < R; ++j) w.h_sys[j].b = const_cast<double*>(eta) + (size_t)j * 8 * C.V;
-    return ws_solve(ctx, c, R, YK_DAGGER, ctx->tol, ctx->tol_mode, ctx->max_iter, precision, stats);
+    return ws_solve(ctx, c, R, YK_DAGGER, ctx->tol, ctx->tol_mode, ctx->max_iter, precision, stats, beside);
 }
 
 // One Langevin step of pion chain c: four coloured noises, the complex solves,
@@ -1311,13 +1316,31 @@ int pion_step(yk_ctx* ctx, int c)
     const int nch = (int)ctx->ch.size();
     const NoiseTables nt = {ctx->d_rows + C.row0, C.nrows, ctx->d_cols + C.col0, C.ncols, ctx->d_white + C.white0,
                             C.nwhite};
-    YK_CK(launch_noise_tables(ctx->d_chains, nt, ctx->max_nx, ctx->max_cols, nullptr, ctx->stream));
-    YK_CK(launch_pion_white(ctx->d_chains + c, C.pi_white, C.V, ctx->stream));
-    for (int a = 0; a < 3; ++a)
-        YK_CK(launch_noise_tables(ctx->d_pchains + (size_t)a * nch, nt, ctx->max_nx, ctx->max_cols,
-                                  C.pi_white + (size_t)a * C.V, ctx->stream));
-    const int rc = pion_solve(ctx, c, 2, nullptr, ctx->precision, nullptr);
-    if (rc && rc != YK_ENOCONV) return rc;
+    auto noise = [&](cudaStream_t q) -> int {
+        YK_CK(launch_noise_tables(ctx->d_chains, nt, ctx->max_nx, ctx->max_cols, nullptr, q));
+        YK_CK(launch_pion_white(ctx->d_chains + c, C.pi_white, C.V, q));
+        for (int a = 0; a < 3; ++a)
+            YK_CK(launch_noise_tables(ctx->d_pchains + (size_t)a * nch, nt, ctx->max_nx, ctx->max_cols,
+                                      C.pi_white + (size_t)a * C.V, q));
+        return YK_OK;
+    };
+    if (C.n_rhs_pion == 0 || !ctx->noise_overlap) {
+        if (int rc = noise(ctx->stream)) return rc;
+        const int rc = pion_solve(ctx, c, 2, nullptr, ctx->precision, nullptr);
+        if (rc && rc != YK_ENOCONV) return rc;
+    } else {
+        // the four noises (thirteen launches) beside the solve, on the SMs it leaves
+        // (64 x 48: 466 us a step with them before it)
+        YK_CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
+        const int rc = pion_solve(ctx, c, 2, nullptr, ctx->precision, nullptr, [&]() -> int {
+            YK_CK(cudaStreamWaitEvent(ctx->aux, ctx->fork_ev, 0));
+            const int nrc = noise(ctx->aux);
+            YK_CK(cudaEventRecord(ctx->join_ev, ctx->aux));
+            YK_CK(cudaStreamWaitEvent(ctx->stream, ctx->join_ev, 0));
+            return nrc;
+        });
+        if (rc && rc != YK_ENOCONV) return rc;
+    }
     const int R = C.n_rhs_pion;
     YK_CK(launch_pion_force(ctx->d_chains + c, C.ws.d_sys, R, C.pi, C.pforce, C.V, ctx->stream));
     YK_CK(launch_pion_drift_update(ctx->d_chains + c, C.pi, C.pforce, C.pdrift, C.pi_xi, C.ptile, C.ptile_f,
