@@ -1018,8 +1018,12 @@ int run_autotune(yk_ctx* ctx)
         T.cg_ms_chosen = std::min(ms[0], ms[1]);
         T.cg_ms_max = std::max(ms[0], ms[1]);
     } else if (ctx->nsys > 1 && !ctx->cg_cluster && ctx->eoc.empty()) {
-        const int maxg = ctx->cg_eo ? cg_eob_max_grid() : cg_max_grid(1, mixed);
-        std::vector<int> cand = {maxg, maxg * 3 / 4, maxg / 2, ctx->n_sm, ctx->n_sm / 2};
+        const int maxg = !ctx->cg_eo ? cg_max_grid(1, mixed)
+                       : ctx->eo_patches ? cg_eop_max_grid(ctx->nsys) : cg_eob_max_grid();
+        // the patch kernel's blocks are a third of an SM's: fewer than one an SM is never
+        // faster, and timing them costs the first step more than the others together
+        std::vector<int> cand = ctx->eo_patches ? std::vector<int>{maxg, maxg * 2 / 3, ctx->n_sm}
+                                                : std::vector<int>{maxg, maxg * 3 / 4, maxg / 2, ctx->n_sm, ctx->n_sm / 2};
         std::sort(cand.begin(), cand.end(), std::greater<int>());
         cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
         cudaEvent_t e0 = nullptr, e1 = nullptr;

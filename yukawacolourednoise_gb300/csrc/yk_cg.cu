@@ -2012,7 +2012,7 @@ __global__ void __launch_bounds__(kHaloThreads) cg_halo_kernel(CGArgs a)
     constexpr int K = 1;
     constexpr int kSkipIm = (1 << 3) | (1 << 5);
     using W = float;
-    extern __shared__ float4 hsm[];
+    extern __shared__ __align__(128) float4 hsm[];
     const int hf = threadIdx.x / kTile, ts = threadIdx.x % kTile;
     __shared__ double red[128];
     __shared__ SysLocal sl[kMaxSysPerBlock];
@@ -2354,6 +2354,27 @@ __device__ __forceinline__ Site<float, 1> eo_sm(const float4* in, int j, int Nh,
                                         diag, r, sp, sm);
 }
 
+// The same in a buffer of rows SB apart, where the x neighbours are j and j + 1 (b)
+// or j - 1 and j.  At r = 1 a time hop keeps one spin entry and the x hops share
+// their sums: 8 operations per spin pair against 14.
+template <bool DAG>
+__device__ __forceinline__ Site<float, 1> eo_hop(const float4* in, int j, int SB, int b, const Site<float, 1>& c, float diag,
+                                                 float r, float sp, float sm)
+{
+    if (r != 1.f) return eo_sm<DAG>(in, j, SB, b, b - 1, c, diag, r, sp, sm);
+    const float4 same = in[j], oth = in[j + 2 * b - 1], up = in[j + SB], dn = in[j - SB];
+    const float e = (b != 0) == DAG ? 1.f : -1.f, h = 0.5f * e;
+    const float a0 = fmaf(-e, same.y, same.x), b0 = fmaf(e, oth.y, oth.x);
+    const float a1 = fmaf(-e, same.w, same.z), b1 = fmaf(e, oth.w, oth.z);
+    const float su = DAG ? sp : sm, sd = DAG ? sm : sp;
+    Site<float, 1> o;
+    o.v[0] = fmaf(-0.5f, a0 + b0, fmaf(-su, DAG ? up.x : dn.x, diag * c.v[0]));
+    o.v[1] = fmaf(h, a0 - b0, fmaf(-sd, DAG ? dn.y : up.y, diag * c.v[1]));
+    o.v[2] = fmaf(-0.5f, a1 + b1, fmaf(-su, DAG ? up.z : dn.z, diag * c.v[2]));
+    o.v[3] = fmaf(h, a1 - b1, fmaf(-sd, DAG ? dn.w : up.w, diag * c.v[3]));
+    return o;
+}
+
 // dirac_combine's hop coefficients in float-float: P = -(r + 1) / 2,
 // M = -(r - 1) / 2, A = -r / 2 (the time hops take +-P and +-M by the
 // antiperiodic signs, the space hops A and +-1/2)
@@ -2433,6 +2454,11 @@ __device__ __forceinline__ SiteFF eo_ff(const double* in, int m, int Ve, int Nh,
 // 512 x 512 lattice's 128 patches are co-resident (its 16 x 16 patches are
 // 512).  PX = 0:
 // whole rows (cg_eo_kernel's first form).
+// A patch's first cell lies kPatchPad cells past a 128-byte line, as the site it
+// copies does (two columns before a multiple of eight): copies of 16 bytes whose
+// sectors lie across the source's cost the staging a twentieth of the iteration
+// (512 x 512: 2573 us a step at 16 bytes off, 2435 so).
+constexpr int kPatchPad = 6;
 __host__ __device__ constexpr int eo_pt(int PX) { return PX == 32 ? 32 : 16; }   // patch rows
 __host__ __device__ constexpr int eo_sr(int PX) { return eo_pt(PX) + 8; }        // staged rows
 __host__ __device__ constexpr int eo_threads(int PX) { return PX == 8 ? 256 : kHaloThreads; }
@@ -2449,7 +2475,7 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
     constexpr int K = 1;
     constexpr int kSkipIm = (1 << 3) | (1 << 5);
     using W = float;
-    extern __shared__ float4 hsm[];
+    extern __shared__ __align__(128) float4 hsm[];
     const int hf = threadIdx.x / kTile, ts = threadIdx.x % kTile;
     __shared__ double red[128];
     __shared__ SysLocal sl[kMaxSysPerBlock];
@@ -2561,7 +2587,7 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
             return (o >= 0 && o < own) ? o : -1;
         }
     };
-    float4* P_st = hsm;                            // p on [0, NB)
+    float4* P_st = hsm + (PATCH ? kPatchPad : 0);   // p on [0, NB)
     float4* R_st = P_st + NB;                      // r there
     float4* A_st = R_st + NB;                      // q there
     float4* X_st = A_st + NB;                      // chi_e increment on the own sites
@@ -3089,15 +3115,21 @@ __device__ bool eob_barrier(const CGArgs& a, unsigned& gen)
 
 // Exclusive prefix over the systems of the tile counts of those whose mode is
 // in `mask` (bit per mode); s_pre[nsys] = the total.  Two systems per thread
-// (blockDim = 512, nsys <= 1024).
+// (NT threads, nsys <= 1024).
+template <int NT>
 __device__ void eob_scan(int nsys, const int* s_mode, const int* s_nt, int mask, int* s_pre)
 {
-    __shared__ int ws[kHaloThreads / 32];
+    constexpr int PER = kEobMaxSystems / NT;
+    __shared__ int ws[NT / 32];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const int q0 = 2 * t, q1 = 2 * t + 1;
-    const int c0 = (q0 < nsys && ((mask >> s_mode[q0]) & 1)) ? s_nt[q0] : 0;
-    const int c1 = (q1 < nsys && ((mask >> s_mode[q1]) & 1)) ? s_nt[q1] : 0;
-    int v = c0 + c1;
+    int c[PER], sum = 0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        const int q = PER * t + i;
+        c[i] = (q < nsys && ((mask >> s_mode[q]) & 1)) ? s_nt[q] : 0;
+        sum += c[i];
+    }
+    int v = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, v, o);
@@ -3106,19 +3138,22 @@ __device__ void eob_scan(int nsys, const int* s_mode, const int* s_nt, int mask,
     if (lane == 31) ws[w] = v;
     __syncthreads();
     if (w == 0) {
-        int x = lane < kHaloThreads / 32 ? ws[lane] : 0;
+        int x = lane < NT / 32 ? ws[lane] : 0;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
-        if (lane < kHaloThreads / 32) ws[lane] = x;
+        if (lane < NT / 32) ws[lane] = x;
     }
     __syncthreads();
-    const int base = (w > 0 ? ws[w - 1] : 0) + v - (c0 + c1);
-    if (q0 < nsys) s_pre[q0] = base;
-    if (q1 < nsys) s_pre[q1] = base + c0;
-    if (t == 0) s_pre[nsys] = ws[kHaloThreads / 32 - 1];
+    int base = (w > 0 ? ws[w - 1] : 0) + v - sum;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+        if (PER * t + i < nsys) s_pre[PER * t + i] = base;
+        base += c[i];
+    }
+    if (t == 0) s_pre[nsys] = ws[NT / 32 - 1];
     __syncthreads();
 }
 
@@ -3235,7 +3270,7 @@ __global__ void __launch_bounds__(kHaloThreads) cg_eob_kernel(CGArgs a)
     // tiles of the systems in `mask`, two tiles at a time (every thread the
     // same trip count: f may hold block-wide barriers).
     auto for_sites = [&](int mask, auto&& f) {
-        eob_scan(nsys, s_mode, s_nt, mask, s_pre);
+        eob_scan<kHaloThreads>(nsys, s_mode, s_nt, mask, s_pre);
         int lo, hi;
         eob_share(s_pre[nsys], &lo, &hi);
         int qc = -1;   // the previous tile's system: a contiguous share mostly stays in one
@@ -3587,33 +3622,36 @@ __global__ void __launch_bounds__(kHaloThreads) cg_eob_kernel(CGArgs a)
 // that iterate are dealt out to the blocks every round, as cg_eob_kernel
 // deals out tiles, and a block takes its share one patch after another: it
 // stages the patch's p, r and q of the previous iteration widened by 4 rows
-// and 2 compact columns, with A_e and 1 / A_o (the next patch's copies in
-// flight while it works on this one), forms p, r, w, v, u and q in shared
+// and 2 compact columns, with A_e and 1 / A_o, forms p, r, w, v, u and q in shared
 // memory, and writes r, p, q, v, the chi increment and the patch's tile
 // partials.  w and u never leave the SM, so a round moves fewer bytes than
 // cg_eob_kernel's four passes, and it has one grid barrier, the reducing
 // one, where cg_eob_kernel has four.  A system's reliable update takes three
 // rounds of its own (kRu: the fold; kRu2: the odd hop; kRu3: the residual and
 // its partials), run site by site beside the other systems' patches, in
-// float-float as in the other even-odd kernels.
+// float-float as in the other even-odd kernels.  A patch is a chain of copies and
+// six passes with a barrier between them, so three 256-thread blocks share an SM,
+// each on a patch of its own (one 512-thread block, the next patch's copies in
+// flight: 91.7 ms for a step of 2 x 1024 x 1024, this 74.3).
 // ---------------------------------------------------------------------------
 constexpr int kEopPT = 32, kEopPX = 16, kEopSW = kEopPX + 4, kEopNB = kEopSW * (kEopPT + 8),
               kEopOwn = kEopPT * kEopPX;
 static_assert(kEopOwn == 2 * kTile, "a patch fills two tiles' partial slots (rows 0-15, 16-31)");
 
-// Shared memory of cg_eop_kernel: two staging sets (p, r, q, A_e, 1 / A_o on
-// the widened patch; the chi increment and v on the own sites), w (then u)
-// and v.
-constexpr size_t kEopSet = 3 * (size_t)kEopNB * sizeof(float4) + 2 * (size_t)kEopNB * sizeof(float) +
-                           2 * (size_t)kEopOwn * sizeof(float4);
-static size_t eop_smem_bytes() { return 2 * kEopSet + 2 * (size_t)kEopNB * sizeof(float4); }
+constexpr int kEopThreads = 256;
+
+// Shared memory of cg_eop_kernel: a widened patch's p, r, q, A_e, 1 / A_o, and ten
+// words a system.
+static size_t eop_smem_bytes(int nsys)
+{
+    return kPatchPad * sizeof(float4) + 3 * (size_t)kEopNB * sizeof(float4) + 2 * (size_t)kEopNB * sizeof(float) +
+           sizeof(int) * (9 * (size_t)nsys + 1);
+}
 
 __device__ __forceinline__ void cp_async4(void* dst, const void* src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-
-__device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 // The reducing barrier of cg_eop_kernel: eob_reduce, with the update's first
 // two rounds (kRu, kRu2: no partials) moving the system to its next round.
@@ -3648,25 +3686,36 @@ __device__ bool eop_reduce(const CGArgs& a, unsigned& gen, int k, double* red, i
     return true;
 }
 
-__global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
+__global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
 {
     constexpr int K = 1;
     constexpr int kSkipIm = (1 << 3) | (1 << 5);
-    constexpr int SB = kEopSW, NB = kEopNB, NT = kHaloThreads;
+    constexpr int SB = kEopSW, NB = kEopNB, NT = kEopThreads;
     using W = float;
-    extern __shared__ float4 hsm[];
-    // staging set s at hsm + s * kEopSet bytes: p, r, q (NB each), xs, v
-    // (own), then A_e, 1 / A_o (NB floats each)
-    auto set_base = [&](int set) -> float4* { return reinterpret_cast<float4*>(reinterpret_cast<char*>(hsm) + set * kEopSet); };
-    float4* Wp = set_base(2);    // w, later u
-    float4* Vp = Wp + NB;        // v
-    const int hf = threadIdx.x / kTile, ts = threadIdx.x % kTile;
+    extern __shared__ __align__(128) float4 hsm[];
+    // the patch's p, r, q (NB each), A_e, 1 / A_o (NB floats each); w (then u) takes
+    // q's place and v that of p, of which its pass reads only the cell it writes;
+    // then the systems' arrays
+    float4* const P_st = hsm + kPatchPad;
+    float4* const R_st = P_st + NB;
+    float4* const A_st = R_st + NB;
+    float* const dep = reinterpret_cast<float*>(A_st + NB);
+    float* const dip = dep + NB;
+    float4* const Wp = A_st;
+    float4* const Vp = P_st;
+    const int ts = threadIdx.x;
     __shared__ double red[128];
-    __shared__ int s_mode[kEobMaxSys], s_par[kEobMaxSys], s_nt[kEobMaxSys], s_t0[kEobMaxSys], s_pre[kEobMaxSys + 1];
-    __shared__ int s_np[kEobMaxSys];   // patches of each system (two tiles each)
-    __shared__ float s_fa[kEobMaxSys], s_fb[kEobMaxSys], s_fc[kEobMaxSys];
-    __shared__ int s_active, s_ru;   // the scalar step's counters (unused here)
     const int nsys = a.sys_count;
+    int* const s_mode = reinterpret_cast<int*>(dip + NB);
+    int* const s_par = s_mode + nsys;
+    int* const s_nt = s_par + nsys;
+    int* const s_t0 = s_nt + nsys;
+    int* const s_np = s_t0 + nsys;    // patches of each system (two tiles each)
+    int* const s_pre = s_np + nsys;   // nsys + 1
+    float* const s_fa = reinterpret_cast<float*>(s_pre + nsys + 1);
+    float* const s_fb = s_fa + nsys;
+    float* const s_fc = s_fb + nsys;
+    __shared__ int s_active, s_ru;   // the scalar step's counters (unused here)
     for (int q = threadIdx.x; q < nsys; q += blockDim.x) {
         const SysDev& S = a.sys[a.sys_first + q];
         s_nt[q] = S.ntiles;
@@ -3721,47 +3770,31 @@ __global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
         return (r >= 0 && r < kEopPT && c >= 0 && c < kEopPX) ? r * kEopPX + c : -1;
     };
 
-    // stage patch P (mode: its system's; kInit: round 0) into set `set`
-    auto stage = [&](const Patch& P, int mode, int set) {
+    // stage patch P (mode: its system's; kInit: round 0)
+    auto stage = [&](const Patch& P, int mode) {
         const SysDev& S = a.sys[a.sys_first + P.q];
         const int cur = s_par[P.q], prv = cur ^ 1;
         const float* Rl = (mode == kRedo || mode == kInit) ? S.r32[cur] : S.r32[prv];
         const float* Pl = mode == kInit ? S.p32[cur] : S.p32[prv];
         const float* Al = prv == 0 ? S.Ap32 : S.t32;
-        float4* B = set_base(set);
-        float4* X = B + 3 * NB;
-        float* D = reinterpret_cast<float*>(X + 2 * kEopOwn);
         for (int j = threadIdx.x; j < NB; j += NT) {
             const int m = buf_m(P, j);
-            cp_async16(B + j, Pl + 4 * (size_t)m);
-            cp_async16(B + NB + j, Rl + 4 * (size_t)m);
-            if (mode == kStep) cp_async16(B + 2 * NB + j, Al + 4 * (size_t)m);
-            cp_async4(D + j, S.diag32 + m);               // A_e (even)
-            cp_async4(D + NB + j, S.diag32 + P.Ve + m);   // 1 / A_o (odd)
+            cp_async16(P_st + j, Pl + 4 * (size_t)m);
+            cp_async16(R_st + j, Rl + 4 * (size_t)m);
+            if (mode == kStep) cp_async16(A_st + j, Al + 4 * (size_t)m);
+            cp_async4(dep + j, S.diag32 + m);               // A_e (even)
+            cp_async4(dip + j, S.diag32 + P.Ve + m);   // 1 / A_o (odd)
         }
-        if (mode == kStep)   // the chi increment and v of the own sites
-            for (int o = threadIdx.x; o < kEopOwn; o += NT) {
-                const int m = own_m(P, o);
-                cp_async16(X + o, S.xs32 + 4 * (size_t)m);
-                cp_async16(X + kEopOwn + o, S.v32 + 4 * (size_t)m);
-            }
         cp_async_commit();
     };
 
-    // the iteration at patch P from staging set `set`
-    auto body = [&](const Patch& P, int mode, int set, bool round0) {
+    // the iteration at the staged patch P
+    auto body = [&](const Patch& P, int mode, bool round0) {
         const SysDev& S = a.sys[a.sys_first + P.q];
-        float4* P_st = set_base(set);
-        float4* R_st = P_st + NB;
-        const float4* A_st = R_st + NB;
-        const float4* X_st = A_st + NB;
-        const float4* Vo_st = X_st + kEopOwn;
-        const float* dep = reinterpret_cast<const float*>(Vo_st + kEopOwn);
-        const float* dip = dep + NB;
         const int cur = s_par[P.q];
         const W rw = (W)S.r;
         const W ar = s_fa[P.q], beta = s_fb[P.q], cre = s_fc[P.q];
-        // A1: p (and r, the chi increment on the own sites) on the buffer
+        // A1: p (and r on the own sites) on the buffer
         for (int j = threadIdx.x; j < NB; j += NT) {
             const int o = own_of(j);
             const Site<W, K> po = ld_sm(P_st, j);
@@ -3773,9 +3806,6 @@ __global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
                 for (int i = 0; i < 4; ++i) p.v[i] = fma(beta, po.v[i], r.v[i]);
                 if (o >= 0) {
                     const int m = own_m(P, o);
-                    Site<W, K> x = ld_sm(X_st, o);
-                    site_axpy<W, K>(x, ar, W(0), ld_sm(Vo_st, o));
-                    YK_ST(W, K, S.xs32, m, x);
                     YK_ST(W, K, S.r32[cur], m, r);
                     YK_ST(W, K, S.p32[cur], m, p);
                     st_sm(R_st, j, r);
@@ -3796,7 +3826,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
         for (int j = SB + threadIdx.x; j < NB - SB; j += NT) {
             const int t = cell_t(P, j), b = (t + 1) & 1;
             const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
-            Site<W, K> h = eo_sm<false>(P_st, j, SB, b, b - 1, zero, W(0), rw, sp, sm);
+            Site<W, K> h = eo_hop<false>(P_st, j, SB, b, zero, W(0), rw, sp, sm);
             const W sc = -dip[j];
 #pragma unroll
             for (int i = 0; i < 4; ++i) h.v[i] *= sc;
@@ -3807,7 +3837,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
         for (int j = 2 * SB + threadIdx.x; j < NB - 2 * SB; j += NT) {
             const int t = cell_t(P, j), b = t & 1;
             const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
-            const Site<W, K> v = eo_sm<false>(Wp, j, SB, b, b - 1, ld_sm(P_st, j), dep[j], rw, sp, sm);
+            const Site<W, K> v = eo_hop<false>(Wp, j, SB, b, ld_sm(P_st, j), dep[j], rw, sp, sm);
             st_sm(Vp, j, v);
             const int o = own_of(j);
             if (o >= 0) YK_ST(W, K, S.v32, own_m(P, o), v);
@@ -3817,7 +3847,7 @@ __global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
         for (int j = 3 * SB + threadIdx.x; j < NB - 3 * SB; j += NT) {
             const int t = cell_t(P, j), b = (t + 1) & 1;
             const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
-            Site<W, K> h = eo_sm<true>(Vp, j, SB, b, b - 1, zero, W(0), rw, sp, sm);
+            Site<W, K> h = eo_hop<true>(Vp, j, SB, b, zero, W(0), rw, sp, sm);
             const W sc = -dip[j];
 #pragma unroll
             for (int i = 0; i < 4; ++i) h.v[i] *= sc;
@@ -3826,76 +3856,82 @@ __global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
         __syncthreads();
         // q = A_e v + H^dag_eo u on the own sites and the patch's partials
         // (round 0 adds |eta|^2 of the compact index's two full sites)
-        FF f[6];
+        for (int hf = 0; hf < kEopOwn / kTile; ++hf) {
+            FF f[6];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) f[i] = FF{0.f, 0.f};
-        const bool on = true;   // rows 0-15 of the patch in threads 0-255, rows 16-31 in 256-511
-        {
-            const int o = hf * kTile + ts;
-            const int j = own_j(o), m = own_m(P, o);
-            const int t = cell_t(P, j), b = t & 1;
-            const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
-            const Site<W, K> v = ld_sm(Vp, j);
-            const Site<W, K> qv = eo_sm<true>(Wp, j, SB, b, b - 1, v, dep[j], rw, sp, sm);
-            YK_ST(W, K, cur == 0 ? S.Ap32 : S.t32, m, qv);
-            const Site<W, K> r = ld_sm(R_st, j);
-            W rq, dummy;
-            site_dot<W, K>(r, qv, rq, dummy);
-            f[0] = FF{site_norm2<W, K>(r), 0.f};
-            f[1] = FF{site_norm2<W, K>(qv), 0.f};
-            f[2] = FF{site_norm2<W, K>(v), 0.f};
-            f[4] = FF{rq, 0.f};
-            if (round0) {
-                const SysDev& SF = a.sys_full[a.sys_first + P.q];
-                const Site<double, K> e0 = load_site<double, K>(SF.b, 2 * m);
-                const Site<double, K> e1 = load_site<double, K>(SF.b, 2 * m + 1);
-                f[5] = ff_of(site_norm2<double, K>(e0) + site_norm2<double, K>(e1));
+            for (int i = 0; i < 6; ++i) f[i] = FF{0.f, 0.f};
+            {
+                const int o = hf * kTile + ts;   // rows 0-15 of the patch, then 16-31
+                const int j = own_j(o), m = own_m(P, o);
+                const int t = cell_t(P, j), b = t & 1;
+                const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
+                const Site<W, K> v = ld_sm(Vp, j);
+                const Site<W, K> qv = eo_hop<true>(Wp, j, SB, b, v, dep[j], rw, sp, sm);
+                YK_ST(W, K, cur == 0 ? S.Ap32 : S.t32, m, qv);
+                const Site<W, K> r = ld_sm(R_st, j);
+                W rq, dummy;
+                site_dot<W, K>(r, qv, rq, dummy);
+                f[0] = FF{site_norm2<W, K>(r), 0.f};
+                f[1] = FF{site_norm2<W, K>(qv), 0.f};
+                f[2] = FF{site_norm2<W, K>(v), 0.f};
+                f[4] = FF{rq, 0.f};
+                if (round0) {
+                    const SysDev& SF = a.sys_full[a.sys_first + P.q];
+                    const Site<double, K> e0 = load_site<double, K>(SF.b, 2 * m);
+                    const Site<double, K> e1 = load_site<double, K>(SF.b, 2 * m + 1);
+                    f[5] = ff_of(site_norm2<double, K>(e0) + site_norm2<double, K>(e1));
+                }
             }
+            const int tile = s_t0[P.q] + 2 * P.lp + hf;
+            if (round0)
+                put_partial_ff<(1 << 3), true>(a, tile, true, f, red);
+            else
+                put_partial_ff<kSkipIm, false>(a, tile, true, f, red);
         }
-        const int tile = s_t0[P.q] + 2 * P.lp + hf;
-        if (round0)
-            put_partial_ff<(1 << 3), true>(a, tile, on, f, red);
-        else
-            put_partial_ff<kSkipIm, false>(a, tile, on, f, red);
     };
 
     // this block's share of the patches of the systems in the pass modes
-    // (round 0: of every system), the next patch's staging in flight
+    // (round 0: of every system)
     auto pass = [&](bool init) {
-        eob_scan(nsys, s_mode, s_np, init ? kAll : kPass, s_pre);
+        eob_scan<NT>(nsys, s_mode, s_np, init ? kAll : kPass, s_pre);
         int lo, hi;
         eob_share(s_pre[nsys], &lo, &hi);
-        int qc = -1, qn = -1;
-        if (lo < hi) {
-            const Patch P0 = patch_of(lo, qn);
-            stage(P0, init ? kInit : s_mode[P0.q], 0);
-        }
+        int qc = -1;
         for (int i = lo; i < hi; ++i) {
-            const int set = (i - lo) & 1;
             const Patch P = patch_of(i, qc);
-            if (i + 1 < hi) {
-                const Patch Pn = patch_of(i + 1, qn);
-                stage(Pn, init ? kInit : s_mode[Pn.q], set ^ 1);
-                cp_async_wait_one();
-            } else {
-                cp_async_wait_all();
+            const int mode = init ? kInit : s_mode[P.q];
+            __syncthreads();   // the previous patch's last reads
+            stage(P, mode);
+            if (mode == kStep) {   // the chi increment on the own sites, while the copies come
+                const SysDev& S = a.sys[a.sys_first + P.q];
+                Site<W, K> xs[kEopOwn / NT], v[kEopOwn / NT];
+#pragma unroll
+                for (int e = 0; e < kEopOwn / NT; ++e) {
+                    const int m = own_m(P, threadIdx.x + e * NT);
+                    xs[e] = YK_LD(W, K, S.xs32, m);
+                    v[e] = YK_LD(W, K, S.v32, m);
+                }
+#pragma unroll
+                for (int e = 0; e < kEopOwn / NT; ++e) {
+                    site_axpy<W, K>(xs[e], s_fa[P.q], W(0), v[e]);
+                    YK_ST(W, K, S.xs32, own_m(P, threadIdx.x + e * NT), xs[e]);
+                }
             }
+            cp_async_wait_all();
             __syncthreads();
-            body(P, init ? kInit : s_mode[P.q], set, init);
+            body(P, mode, init);
         }
     };
 
     // Runs f(S, q, m, tile, tile_on, on) for every site of this block's share
-    // of the tiles of the systems in `mask`, two tiles at a time.
+    // of the tiles of the systems in `mask`.
     auto for_sites = [&](int mask, auto&& f) {
-        eob_scan(nsys, s_mode, s_nt, mask, s_pre);
+        eob_scan<NT>(nsys, s_mode, s_nt, mask, s_pre);
         int lo, hi;
         eob_share(s_pre[nsys], &lo, &hi);
         int qc = -1;
-        for (int base = lo; base < hi; base += 2) {
-            const int i = base + hf;
-            const bool tile_on = i < hi;
-            const int ii = tile_on ? i : lo;
+        for (int ii = lo; ii < hi; ++ii) {
+            const bool tile_on = true;
             const int q = (qc >= 0 && ii >= s_pre[qc] && ii < s_pre[qc + 1]) ? qc : eob_find(ii, nsys, s_pre);
             qc = q;
             const int lt = ii - s_pre[q];
@@ -4078,10 +4114,11 @@ __global__ void __launch_bounds__(kHaloThreads, 1) cg_eop_kernel(CGArgs a)
 
 // Shared memory of cg_eo_kernel for `own` compact sites per block and a
 // staged buffer of nb cells: p, r, q, w (then u) and v on the buffer, the chi
-// increment and v on the own sites, A_e and 1 / A_o in FP32 on the buffer.
-static size_t eo_smem_bytes(int own, int nb)
+// increment and v on the own sites, A_e and 1 / A_o in FP32 on the buffer; `pad`
+// cells before them.
+static size_t eo_smem_bytes(int own, int nb, int pad = 0)
 {
-    return (5 * (size_t)nb + 2 * (size_t)own) * sizeof(float4) + 2 * (size_t)nb * sizeof(float);
+    return (pad + 5 * (size_t)nb + 2 * (size_t)own) * sizeof(float4) + 2 * (size_t)nb * sizeof(float);
 }
 
 // Failure detection without a fault: block 0 waits through nsync on block
@@ -4238,7 +4275,7 @@ static bool eo_patch_takes(int Nt, int Nx, int* patches, size_t* smem)
     constexpr int PT = eo_pt(PX);
     if (Nt < PT || Nx < 2 * PX || (Nt % PT) || (Nx % (2 * PX))) return false;
     *patches = (Nt / PT) * (Nx / (2 * PX));
-    *smem = eo_smem_bytes(PT * PX, eo_sw(PX) * eo_sr(PX));
+    *smem = eo_smem_bytes(PT * PX, eo_sw(PX) * eo_sr(PX), kPatchPad);
     return *smem <= kHaloMaxSmem;
 }
 
@@ -4263,7 +4300,7 @@ static int eo_patch_max_grid()
 {
     static int maxg = -1;
     if (maxg < 0) {
-        const int smem = (int)eo_smem_bytes(eo_pt(PX) * PX, eo_sw(PX) * eo_sr(PX));
+        const int smem = (int)eo_smem_bytes(eo_pt(PX) * PX, eo_sw(PX) * eo_sr(PX), kPatchPad);
         cudaFuncSetAttribute((const void*)cg_eo_kernel<PX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int dev = 0, nsm = 0, per = 0;
         cudaGetDevice(&dev);
@@ -4289,24 +4326,20 @@ static int eob_max_grid()
     return maxg;
 }
 
-static int eop_max_grid()
+static int eop_max_grid(int nsys)
 {
-    static int maxg = -1;
-    if (maxg < 0) {
-        const int smem = (int)eop_smem_bytes();
-        cudaFuncSetAttribute((const void*)cg_eop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        int dev = 0, nsm = 0, per = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)cg_eop_kernel, kHaloThreads, smem) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            per = 0;
-        }
-        maxg = per * nsm;
-        if (maxg > kMaxGrid) maxg = kMaxGrid;
+    const int smem = (int)eop_smem_bytes(nsys);
+    static const bool ok = cudaFuncSetAttribute((const void*)cg_eop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                (int)eop_smem_bytes(kEobMaxSys)) == cudaSuccess;
+    int dev = 0, nsm = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (!ok || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, (const void*)cg_eop_kernel, kEopThreads, smem) !=
+                   cudaSuccess) {
+        cudaGetLastError();
+        per = 0;
     }
-    return maxg;
+    return std::min(per * nsm, kMaxGrid);
 }
 
 static int halo_max_grid()
@@ -4325,6 +4358,8 @@ static int halo_max_grid()
 
 int cg_eob_max_grid() { return eob_max_grid(); }
 
+int cg_eop_max_grid(int nsys) { return eop_max_grid(nsys); }
+
 void cg_halo_init()
 {
     halo_max_grid();
@@ -4333,7 +4368,7 @@ void cg_halo_init()
     eo_patch_max_grid<8>();
     eo_patch_max_grid<32>();
     eob_max_grid();
-    eop_max_grid();
+    eop_max_grid(1);
 }
 
 static int capped(int maxg, int cap) { return cap > 0 && cap < maxg ? cap : maxg; }
@@ -4351,7 +4386,7 @@ int cg_predict_grid(const CGArgs& a, bool mixed, const OneLattice& lat)
         if (eo_single_variant(a, &px, &eg, &etpb, &es)) return eg;
         const int nt = a.eo_tile_end - a.eo_tile_begin;
         const char* pe = getenv("YK_CG_EOP");
-        if (a.eo_patches && !(pe && pe[0] == '0') && eop_max_grid() > 0) return std::min(capped(eop_max_grid(), a.grid_cap), std::max(nt, 1));
+        if (a.eo_patches && !(pe && pe[0] == '0') && eop_max_grid(a.sys_count) > 0) return std::min(capped(eop_max_grid(a.sys_count), a.grid_cap), std::max(nt, 1));
         return std::min(capped(eob_max_grid(), a.grid_cap), std::max((nt + 1) / 2, 1));
     }
     if (const int g = cg_small_grid(a, 1, mixed, lat)) return g;
@@ -4459,8 +4494,8 @@ static cudaError_t launch_cg_t(const CGArgs& a0, cudaStream_t stream, int* grid_
             // lattices that 16 x 16 patches tile: the batched patch kernel
             // (YK_CG_EOP=0: the four-pass kernel below), one block per SM
             const char* pe = getenv("YK_CG_EOP");
-            if (a.eo_patches && !(pe && pe[0] == '0') && eop_max_grid() > 0) {
-                int pg = capped(eop_max_grid(), a.grid_cap);
+            if (a.eo_patches && !(pe && pe[0] == '0') && eop_max_grid(a.sys_count) > 0) {
+                int pg = capped(eop_max_grid(a.sys_count), a.grid_cap);
                 const int want = a.eo_tile_end - a.eo_tile_begin;   // patches (one tile each)
                 if (pg > want) pg = want;
                 if (pg < 1) pg = 1;
@@ -4471,8 +4506,8 @@ static cudaError_t launch_cg_t(const CGArgs& a0, cudaStream_t stream, int* grid_
                 cg_prepare_kernel<<<1, 256, 0, stream>>>(e);
                 cudaLaunchConfig_t cfg = {};
                 cfg.gridDim = dim3(pg);
-                cfg.blockDim = dim3(kHaloThreads);
-                cfg.dynamicSmemBytes = eop_smem_bytes();
+                cfg.blockDim = dim3(kEopThreads);
+                cfg.dynamicSmemBytes = eop_smem_bytes(a.sys_count);
                 cfg.stream = stream;
                 cudaLaunchAttribute attr[1];
                 attr[0].id = cudaLaunchAttributeCooperative;

@@ -50,6 +50,7 @@ cudaError_t launch_cg_balance(const CGArgs& a, int grid, int* out, cudaStream_t 
 // Largest co-resident grid of the CG kernel (cached; call before capturing).
 int cg_max_grid(int K, bool mixed);
 int cg_eob_max_grid();   // co-resident blocks of the batched even-odd CG
+int cg_eop_max_grid(int nsys);   // of the batched patch kernel for that many systems
 // Kernel attributes and occupancy of the halo CG kernel (call before any stream capture).
 void cg_halo_init();
 // Runs the wait-timeout probe kernel on `stream`; *status = the device status
