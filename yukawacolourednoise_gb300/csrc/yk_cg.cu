@@ -252,6 +252,26 @@ __device__ __forceinline__ int fix_value_of_slot(int i)
     return i == 0 ? 0 : i == 1 ? 1 : i == 2 ? 2 : i == 4 ? 3 : -1;
 }
 
+// Slots: the same sums without the atomics and the arrival counter.  A block
+// publishes its sum of each value in a word of its own, in the second half of its
+// neighbour flag's line, and every block reads every word: the load that finds the
+// block arrived has read its sum.  The sums order no other memory (the vectors'
+// neighbours are told by the flag, whose release waits for the block's writes
+// meanwhile).  A word is the sum times four and a tag of 1 to 3 (zero: none yet): the
+// two buffers alternate and a buffer's tag changes with each use, so no word of an
+// earlier barrier is taken for one of this.  (A block writes a buffer again only
+// after a barrier that every reader of it has reached.)
+constexpr int kSlotWord = 8;                    // 8-byte words into the flag's line
+constexpr long long kSlotOver = -(1ll << 61);   // in a sum's place: a value was too large
+static_assert(8 * (kSlotWord + 8) <= 4 * kFlagStride, "both buffers' four words in a flag's line");
+
+__device__ __forceinline__ unsigned long long* slot_word(unsigned* flags, int block, unsigned sgen, int c)
+{
+    return reinterpret_cast<unsigned long long*>(flags + (size_t)block * kFlagStride) + kSlotWord + 4 * (sgen & 1u) + c;
+}
+
+__device__ __forceinline__ unsigned slot_tag(unsigned sgen) { return 1u + (sgen >> 1) % 3u; }
+
 // Blocks holding stencil neighbours of this block's sites.
 struct Deps {
     int n;
@@ -267,6 +287,56 @@ __device__ __forceinline__ bool wait_over(long long t0, int* err)
         return true;
     }
     return *(volatile int*)err != 0;
+}
+
+// The slots' sums, by one warp: value c in lanes c, c + 4, ...; kFixLimit where a
+// block's value was too large.  False when a wait gave up.
+__device__ __forceinline__ bool slot_sums(const CGArgs& a, unsigned sgen, long long& sum)
+{
+    constexpr int U = 8;   // loads in flight
+    const unsigned tag = slot_tag(sgen);
+    const int lane = threadIdx.x & 31, nb = (int)gridDim.x;
+    const long long t0 = clock64();
+    long long s0 = 0, s1 = 0;
+    bool over = false, late = false;
+    unsigned polls = 0;
+    for (int base = lane / 2; base < nb; base += 16 * U) {
+        unsigned todo = 0;   // of the U blocks base, base + 16, ...
+#pragma unroll
+        for (int i = 0; i < U; ++i) todo |= (base + 16 * i < nb ? 1u : 0u) << i;
+        while (todo && !late) {
+            unsigned long long x[U], y[U];
+#pragma unroll
+            for (int i = 0; i < U; ++i) {
+                x[i] = y[i] = 0;
+                if ((todo >> i) & 1u)
+                    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];"
+                                 : "=l"(x[i]), "=l"(y[i])
+                                 : "l"(slot_word(a.flags, base + 16 * i, sgen, 2 * (lane & 1)))
+                                 : "memory");
+            }
+#pragma unroll
+            for (int i = 0; i < U; ++i)
+                if ((unsigned)(x[i] & 3u) == tag && (unsigned)(y[i] & 3u) == tag) {
+                    const long long vx = (long long)x[i] >> 2, vy = (long long)y[i] >> 2;
+                    over |= vx == kSlotOver || vy == kSlotOver;
+                    s0 += vx;
+                    s1 += vy;
+                    todo &= ~(1u << i);
+                }
+            if (todo && (++polls & 15) == 0) late = wait_over(t0, a.err);
+        }
+    }
+    if (__any_sync(0xffffffffu, late)) return false;
+#pragma unroll
+    for (int o = 16; o >= 2; o >>= 1) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    }
+    // lanes 0 and 1 hold values 0, 1 and 2, 3
+    const long long e = __shfl_sync(0xffffffffu, s0, (lane >> 1) & 1), f = __shfl_sync(0xffffffffu, s1, (lane >> 1) & 1);
+    sum = __any_sync(0xffffffffu, over) ? kFixLimit : (lane & 1) ? f : e;
+    return true;
 }
 
 __device__ __forceinline__ unsigned ld_acquire_flag(const unsigned* p)
@@ -1160,148 +1230,186 @@ __device__ void sum_partials(const CGArgs& a, int tile0, int ntiles, double* red
 // (the other blocks' writes of the pass are visible), before the scalar
 // work: the halo kernel issues the next pass's loads there.
 struct NoHook {
-    __device__ void operator()() const {}
+    __device__ int operator()(bool) const { return 0; }
 };
 
 // RUFIX: the caller's reliable updates add their partials to the fixed-point
 // totals too (put_partial_ff RU_SCALE), so an update round may take the fast
 // path (fast_ru_step) like an ordinary one.
-template <int K, bool MIXED, bool RUFIX = false, typename Hook = NoHook>
+// SLOTS: an iteration whose scales hold came through put_slots (sgen counts those
+// barriers, gen the others) where the caller says `slots`: warp 0 takes the sums and the step while the other warps
+// wait for the neighbours and start the copies, in the hook.  (512 x 512, a step: 2435 us
+// with the counted barrier and four atomics a tile, 2222 so.)
+template <int K, bool MIXED, bool RUFIX = false, bool SLOTS = false, typename Hook = NoHook>
 __device__ __forceinline__ bool solo_reduce_body(const CGArgs& a, unsigned& gen, int k, bool ru_round, double* red,
                                                  CGState& lst, SysLocal& L, int* s_nact, int* s_anyru, int* s_cnt,
-                                                 int* esc, int* s_fast, FastShadow& fs, Hook after_barrier = Hook())
+                                                 int* esc, int* s_fast, FastShadow& fs, unsigned& sgen, bool slots,
+                                                 Hook after_barrier = Hook())
 {
     constexpr bool kFix = MIXED && K == 1;   // fixed-point sums available
-    int bad = 0;   // thread 0: its wait gave up
-#ifdef YK_CG_TIMING
-    long long ql = clock64();
-#endif
-    __syncthreads();
-#ifdef YK_CG_TIMING
-    const long long q0 = clock64();
-#endif
-    YK_QMARK(0);
-    if (threadIdx.x == 0) {
-        if (kFix && blockIdx.x == 0) {
-            // the buffer of the barrier after this one: nobody reads it any more
-            // (its last readers arrived here already) and nobody adds to it
-            // before this block has arrived
-            long long (*z)[16] = a.bar->fsum[(gen + 2u) % 3u];
-            for (int c = 0; c < 4; ++c) z[c][0] = 0;
-            z[0][kFixOverflowWord] = 0;
-        }
-        arrive_release(&a.bar->arrive);
-        YK_QMARK(1);
-        const unsigned target = gridDim.x * (gen + 1u);
-        const long long t0 = clock64();
-        while ((int)(ld_acquire(&a.bar->arrive) - target) < 0)
-            if (wait_over(t0, a.err)) {
-                bad = 1;
-                break;
-            }
-        YK_QMARK(2);
-        s_cnt[0] = 0;
-        s_cnt[1] = 0;
-    }
-    ++gen;
-    if (__syncthreads_or(bad)) return false;
-    // the fixed-point totals of this barrier, if the tiles added them: lanes
-    // 0-3 load one each, lane 4 the overflow flag -- ahead of the hook's loads
-    const bool fix_now = kFix && (!ru_round || RUFIX) && *s_fast;
-    long long Sv = 0;
-    unsigned long long over_v = 0ull;
-    if (fix_now && threadIdx.x < 5) {
-        const long long(*f)[16] = a.bar->fsum[gen % 3u];
-        if (threadIdx.x < 4)
-            Sv = (long long)ld_word(reinterpret_cast<const unsigned long long*>(&f[threadIdx.x][0]));
-        else
-            over_v = ld_word(reinterpret_cast<const unsigned long long*>(&f[0][kFixOverflowWord]));
-    }
-    after_barrier();
-    YK_QMARK(3);
+    // sums in fixed point, if the tiles added them
+    const bool fix_now = !slots && kFix && (!ru_round || RUFIX) && *s_fast;
     double s[6];
-#ifdef YK_CG_TIMING
-    const long long q1 = clock64();
-#endif
-    // fixed-point totals of this barrier, if the tiles added them
     bool fast = false, stepped = false;
     int s_scales = 0;   // thread 0: 2 = next scales set from the integer totals
     __shared__ int s_dec;   // thread 0's verdict on the fixed-point totals (0 none, 1 sums, 2 stepped)
-    if constexpr (kFix) {
-        if (fix_now) {
-            if (threadIdx.x < 32) {
-                // lanes 0-3: one total each (load, range check, conversion,
-                // next scale); lane 4: the overflow flag; lane 5: the
-                // periodic trigger; lane 0 then steps
-                const unsigned full = 0xffffffffu;
-                const int lane = threadIdx.x;
-                bool okl = true, conv = true;
-                FF fv = {0.f, 0.f};
-                int er = 0, due = 0;
-                // an update's <r, p> (lane 2) is at the scale of |r|^2
-                const int el = (ru_round && lane == 2) ? esc[0] : (lane < 4 ? esc[lane] : 0);
-                if (lane < 4) {
-                    okl = Sv < kFixLimit && Sv > -kFixLimit;
-                    conv = okl && fix_to_ff(Sv, el, fv);
-                    if (lane < 3 && Sv > 0) er = fix_rescale(Sv, el);
-                } else if (lane == 4) {
-                    okl = over_v == 0ull;
-                } else if (lane == 5) {
-                    due = a.reliable_every > 0 && (k + 1) % a.reliable_every == 0;
-                }
-                const bool ok = __all_sync(full, okl);
-                const bool convall = __all_sync(full, conv);
-                const bool pos = __all_sync(full, (ru_round ? lane != 0 : lane >= 3) || Sv > 0);
-                FF v[4];
-                long long S[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    v[c] = FF{__shfl_sync(full, fv.hi, c), __shfl_sync(full, fv.lo, c)};
-                    S[c] = __shfl_sync(full, Sv, c);
-                }
-                const int e0 = __shfl_sync(full, er, 0), e1 = __shfl_sync(full, er, 1), e2 = __shfl_sync(full, er, 2);
-                due = __shfl_sync(full, due, 5);
-                YK_QMARK(4);
-                __syncwarp();   // every lane has read esc
-                if (lane == 0) {
-                    bool done = false;
-                    if (ok) {
-                        // the ordinary step on the FP32 pipes; the FP64 one otherwise
-                        done = convall && lst.mode != kIdle &&
-                               (ru_round ? fast_ru_step(a, k, v[0], v[2], lst, L)
-                                         : fast_step(a, k, v[0], v[1], v[2], v[3], due != 0, lst, fs, L));
-                        if (!done) {
-                            s[0] = scalbn((double)S[0], -esc[0]);
-                            s[1] = scalbn((double)S[1], -esc[1]);
-                            s[2] = scalbn((double)S[2], -(ru_round ? esc[0] : esc[2]));
-                            s[4] = scalbn((double)S[3], -esc[3]);
-                            s[3] = s[5] = 0.0;
-                        }
-                        // next scales straight from the integer totals (an
-                        // update's round renews the |r|^2 scale only)
-                        if (pos) {
-                            esc[0] = e0;
-                            if (!ru_round) {
-                                esc[1] = e1;
-                                esc[2] = e2;
-                                esc[3] = (e0 + e1) / 2 - 1;   // |<r, Ap>| <= |r| |Ap|
-                            }
-                            s_scales = 2;   // scales already set
-                        } else {
-                            s_scales = 3;   // no usable scales: the next sums go through the tile partials
-                        }
-                    }
-                    s_dec = ok ? (done ? 2 : 1) : 0;
-                    if (done) {
-                        // the block's state for the next pass, before the
-                        // barrier that publishes the step
-                        *s_nact = 1;
-                        *s_anyru = lst.mode == kRu;
-                        *s_fast = s_scales == 2 ? 1 : 0;
-                    }
-                    YK_QMARK(5);
-                }
+#ifdef YK_CG_TIMING
+    long long ql = clock64();
+    const long long q0 = ql;
+    long long q1 = ql;
+#endif
+    // warp 0: the fixed-point totals (value c in lane c) and the overflow flag (lane 4)
+    auto decide = [&](long long Sv, unsigned long long over_v) {
+        if constexpr (kFix) {
+            // lanes 0-3: one total each (load, range check, conversion,
+            // next scale); lane 4: the overflow flag; lane 5: the
+            // periodic trigger; lane 0 then steps
+            const unsigned full = 0xffffffffu;
+            const int lane = threadIdx.x;
+            bool okl = true, conv = true;
+            FF fv = {0.f, 0.f};
+            int er = 0, due = 0;
+            // an update's <r, p> (lane 2) is at the scale of |r|^2
+            const int el = (ru_round && lane == 2) ? esc[0] : (lane < 4 ? esc[lane] : 0);
+            if (lane < 4) {
+                okl = Sv < kFixLimit && Sv > -kFixLimit;
+                conv = okl && fix_to_ff(Sv, el, fv);
+                if (lane < 3 && Sv > 0) er = fix_rescale(Sv, el);
+            } else if (lane == 4) {
+                okl = over_v == 0ull;
+            } else if (lane == 5) {
+                due = a.reliable_every > 0 && (k + 1) % a.reliable_every == 0;
             }
+            const bool ok = __all_sync(full, okl);
+            const bool convall = __all_sync(full, conv);
+            const bool pos = __all_sync(full, (ru_round ? lane != 0 : lane >= 3) || Sv > 0);
+            FF v[4];
+            long long S[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                v[c] = FF{__shfl_sync(full, fv.hi, c), __shfl_sync(full, fv.lo, c)};
+                S[c] = __shfl_sync(full, Sv, c);
+            }
+            const int e0 = __shfl_sync(full, er, 0), e1 = __shfl_sync(full, er, 1), e2 = __shfl_sync(full, er, 2);
+            due = __shfl_sync(full, due, 5);
+            YK_QMARK(4);
+            __syncwarp();   // every lane has read esc
+            if (lane == 0) {
+                bool done = false;
+                if (ok) {
+                    // the ordinary step on the FP32 pipes; the FP64 one otherwise
+                    done = convall && lst.mode != kIdle &&
+                           (ru_round ? fast_ru_step(a, k, v[0], v[2], lst, L)
+                                     : fast_step(a, k, v[0], v[1], v[2], v[3], due != 0, lst, fs, L));
+                    if (!done) {
+                        s[0] = scalbn((double)S[0], -esc[0]);
+                        s[1] = scalbn((double)S[1], -esc[1]);
+                        s[2] = scalbn((double)S[2], -(ru_round ? esc[0] : esc[2]));
+                        s[4] = scalbn((double)S[3], -esc[3]);
+                        s[3] = s[5] = 0.0;
+                    }
+                    // next scales straight from the integer totals (an
+                    // update's round renews the |r|^2 scale only)
+                    if (pos) {
+                        esc[0] = e0;
+                        if (!ru_round) {
+                            esc[1] = e1;
+                            esc[2] = e2;
+                            esc[3] = (e0 + e1) / 2 - 1;   // |<r, Ap>| <= |r| |Ap|
+                        }
+                        s_scales = 2;   // scales already set
+                    } else {
+                        s_scales = 3;   // no usable scales: the next sums go through the tile partials
+                    }
+                }
+                s_dec = ok ? (done ? 2 : 1) : 0;
+                if (done) {
+                    // the block's state for the next pass, before the
+                    // barrier that publishes the step
+                    *s_nact = 1;
+                    *s_anyru = lst.mode == kRu;
+                    *s_fast = s_scales == 2 ? 1 : 0;
+                }
+                YK_QMARK(5);
+            }
+        }
+    };
+    // arrive and wait for every block; false when a wait gave up
+    auto counted = [&]() -> bool {
+        int bad = 0;
+        __syncthreads();
+        YK_QMARK(0);
+        if (threadIdx.x == 0) {
+            if (kFix && blockIdx.x == 0) {
+                // the buffer of the barrier after this one: nobody reads it any more
+                // (its last readers arrived here already) and nobody adds to it
+                // before this block has arrived
+                long long (*z)[16] = a.bar->fsum[(gen + 2u) % 3u];
+                for (int c = 0; c < 4; ++c) z[c][0] = 0;
+                z[0][kFixOverflowWord] = 0;
+            }
+            arrive_release(&a.bar->arrive);
+            YK_QMARK(1);
+            const unsigned target = gridDim.x * (gen + 1u);
+            const long long t0 = clock64();
+            while ((int)(ld_acquire(&a.bar->arrive) - target) < 0)
+                if (wait_over(t0, a.err)) {
+                    bad = 1;
+                    break;
+                }
+            YK_QMARK(2);
+            s_cnt[0] = 0;
+            s_cnt[1] = 0;
+        }
+        ++gen;
+        return !__syncthreads_or(bad);
+    };
+    if (SLOTS && slots) {
+        int bad = 0;
+        if (threadIdx.x < 32) {
+            long long Sv;
+            bad = !slot_sums(a, sgen, Sv);
+            YK_QMARK(2);
+            if (threadIdx.x == 0) {
+                s_cnt[0] = 0;
+                s_cnt[1] = 0;
+            }
+            if (!bad) decide(Sv, 0ull);
+        }
+        bad |= after_barrier(true);
+        ++sgen;
+        if (__syncthreads_or(bad)) return false;
+        fast = s_dec != 0;
+        stepped = s_dec == 2;
+        if (stepped) {
+            YK_QMARK(6);
+#ifdef YK_CG_TIMING
+            if (threadIdx.x == 0 && blockIdx.x == 0) atomicAdd(&g_cg_f[3], 1ull);
+#endif
+            return true;
+        }
+        // the tiles' partials, for which the slots did not wait
+        if (!fast && !counted()) return false;
+    } else {
+        if (!counted()) return false;
+        // the fixed-point totals of this barrier, if the tiles added them: lanes
+        // 0-3 load one each, lane 4 the overflow flag -- ahead of the hook's loads
+        long long Sv = 0;
+        unsigned long long over_v = 0ull;
+        if (fix_now && threadIdx.x < 5) {
+            const long long(*f)[16] = a.bar->fsum[gen % 3u];
+            if (threadIdx.x < 4)
+                Sv = (long long)ld_word(reinterpret_cast<const unsigned long long*>(&f[threadIdx.x][0]));
+            else
+                over_v = ld_word(reinterpret_cast<const unsigned long long*>(&f[0][kFixOverflowWord]));
+        }
+        after_barrier(false);
+        YK_QMARK(3);
+#ifdef YK_CG_TIMING
+        q1 = clock64();
+#endif
+        if (fix_now) {
+            if (threadIdx.x < 32) decide(Sv, over_v);
             // s_dec is written again only after the barriers of the passes that follow
             __syncthreads();
             fast = s_dec != 0;
@@ -1390,7 +1498,8 @@ __device__ __noinline__ bool solo_reduce(const CGArgs& a, unsigned& gen, int k, 
                                          SysLocal& L, int* s_nact, int* s_anyru, int* s_cnt, int* esc, int* s_fast,
                                          FastShadow& fs)
 {
-    return solo_reduce_body<K, MIXED>(a, gen, k, ru_round, red, lst, L, s_nact, s_anyru, s_cnt, esc, s_fast, fs);
+    unsigned sgen = 0;
+    return solo_reduce_body<K, MIXED>(a, gen, k, ru_round, red, lst, L, s_nact, s_anyru, s_cnt, esc, s_fast, fs, sgen, false);
 }
 
 template <typename W, bool MIXED>
@@ -1580,6 +1689,96 @@ __device__ __forceinline__ void put_partial_ff(const CGArgs& a, int tile, bool w
             }
         }
     }
+}
+
+// A warp's FP32 sums of NV values (4 or 8), the butterfly's: each step leaves every
+// lane half of the values, so 8 take 9 shuffles (put_partial_ff's way 40).  Returns
+// the sum of value lane / (32 / NV).
+template <int NV>
+__device__ __forceinline__ float warp_sums(float (&v)[NV])
+{
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = NV / 2; n > 0; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < n; ++i) {
+            const float got = __shfl_xor_sync(0xffffffffu, up ? v[i] : v[i + n], o);
+            v[i] = (up ? v[i + n] : v[i]) + got;
+        }
+    }
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+// Value c's partial slots of T tiles from `tile0` on, by one warp, from the warps'
+// sums s_w[tile][value][warp] by put_partial_ff's tree.
+template <int T>
+__device__ __forceinline__ void tile_partials(const CGArgs& a, int tile0, int c, const float* s_w)
+{
+    constexpr int hw = kTile / 32;
+    const int lane = threadIdx.x & 31, tl = lane / hw, u = lane % hw;
+    FF t{tl < T ? s_w[(tl * 4 + c) * hw + u] : 0.f, 0.f};
+#pragma unroll
+    for (int q = hw / 2; q > 0; q >>= 1) t = ff_add(t, ff_shfl_xor(t, q));
+    if (tl < T) {
+        float2* part = a.partial[tile0 + tl].f;
+        if (u == 0)
+            part[c == 3 ? 4 : c] = make_float2(t.hi, t.lo);
+        else if (c == 3 && u < 3)
+            part[u == 1 ? 3 : 5] = make_float2(0.f, 0.f);
+    }
+}
+
+// The single-system patch kernel's sums of an iteration whose fixed-point scales
+// hold: the four values of the block's T tiles (f[4 i + c]: of tile tb + half + 2 i at
+// this thread's site).  The warps' sums go into fixed point as they are, and warp 0
+// adds them and publishes the block's words.  Meanwhile the last warp tells the
+// neighbours (flag: `epoch`) and four others keep the tiles' partial slots, for sums
+// that come out too large.
+template <int T, int R, int NT>
+__device__ __forceinline__ void put_slots(const CGArgs& a, int tb, float (&f)[4 * R], double* red, const int* esc,
+                                          unsigned epoch, unsigned sgen)
+{
+    constexpr int hw = kTile / 32, NV = 4 * R, NW = NT / 32;
+    static_assert(NW == 8 || NW == 16, "eight lanes a value add the warps' sums");
+    float* const s_w = reinterpret_cast<float*>(red);                        // T x 4 x hw
+    long long* const s_fx = reinterpret_cast<long long*>(red) + 2 * hw * 4;  // 4 x NW
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, half = threadIdx.x / kTile;
+    const float v = warp_sums<NV>(f);
+    constexpr int rest = 32 / NV;   // lanes that hold the same value
+    const int val = lane / rest, c = val % 4, tile_of = half + 2 * (val / 4);
+    if (lane % rest == 0 && tile_of < T) s_w[(tile_of * 4 + c) * hw + w % hw] = v;
+    long long x = f2fix(v, esc[c]);
+    const long long lim = fix_tile_limit(a.tile_end - a.tile_begin) / hw;
+    const bool over = !(x < lim && x > -lim);
+    if constexpr (R == 2) x += __shfl_xor_sync(0xffffffffu, x, 16);
+    if (__any_sync(0xffffffffu, over)) x = kSlotOver;
+    if (lane % rest == 0 && val < 4) s_fx[c * NW + w] = x;
+    __syncthreads();
+    if (w == 0) {
+        const int cc = lane / 8, u = lane % 8;
+        long long s = s_fx[cc * NW + u];
+        bool ov = s == kSlotOver;
+        if constexpr (NW == 16) {
+            const long long s2 = s_fx[cc * NW + u + 8];
+            ov |= s2 == kSlotOver;
+            s += s2;
+        }
+#pragma unroll
+        for (int q = 4; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+        if (__any_sync(0xffffffffu, ov)) s = kSlotOver;
+        if (u == 0)
+            asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(slot_word(a.flags, blockIdx.x, sgen, cc)),
+                         "l"(((unsigned long long)s << 2) | slot_tag(sgen))
+                         : "memory");
+    } else if (w == NW - 1 && lane == 0) {
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.flags + (size_t)blockIdx.x * kFlagStride), "r"(epoch)
+                     : "memory");
+    }
+    __syncwarp();
+    if (w >= 2 && w < 6) tile_partials<T>(a, tb, w - 2, s_w);
 }
 
 // Reliable update (mixed solver), first part, at one site of a system in
@@ -2169,13 +2368,15 @@ __global__ void __launch_bounds__(kHaloThreads) cg_halo_kernel(CGArgs a)
     auto reduce = [&](int kk, bool ru) -> bool {
         // once the barrier of an ordinary iteration is passed, stage the next
         // one on the guess that it is an ordinary step too
-        auto prefetch = [&]() {
-            if (ru) return;
+        auto prefetch = [&](bool) -> int {
+            if (ru) return 0;
             const int k1 = kk + 1;
             stage(kStep, k1 & 1, (k1 & 1) ^ 1);
             staged_k = k1;
+            return 0;
         };
-        return solo_reduce_body<K, true>(sa, gen, kk, ru, red, lst, sl[0], &s_nact, &s_anyru, s_cnt, s_esc, &s_fast, fsh,
+        unsigned sgen = 0;
+        return solo_reduce_body<K, true>(sa, gen, kk, ru, red, lst, sl[0], &s_nact, &s_anyru, s_cnt, s_esc, &s_fast, fsh, sgen, false,
                                          prefetch);
     };
 
@@ -2352,27 +2553,6 @@ __device__ __forceinline__ Site<float, 1> eo_sm(const float4* in, int j, int Nh,
 {
     return dirac_combine<float, 1, DAG>(c, ld_sm(in, j + Nh), ld_sm(in, j - Nh), ld_sm(in, j + dxu), ld_sm(in, j + dxd),
                                         diag, r, sp, sm);
-}
-
-// The same in a buffer of rows SB apart, where the x neighbours are j and j + 1 (b)
-// or j - 1 and j.  At r = 1 a time hop keeps one spin entry and the x hops share
-// their sums: 8 operations per spin pair against 14.
-template <bool DAG>
-__device__ __forceinline__ Site<float, 1> eo_hop(const float4* in, int j, int SB, int b, const Site<float, 1>& c, float diag,
-                                                 float r, float sp, float sm)
-{
-    if (r != 1.f) return eo_sm<DAG>(in, j, SB, b, b - 1, c, diag, r, sp, sm);
-    const float4 same = in[j], oth = in[j + 2 * b - 1], up = in[j + SB], dn = in[j - SB];
-    const float e = (b != 0) == DAG ? 1.f : -1.f, h = 0.5f * e;
-    const float a0 = fmaf(-e, same.y, same.x), b0 = fmaf(e, oth.y, oth.x);
-    const float a1 = fmaf(-e, same.w, same.z), b1 = fmaf(e, oth.w, oth.z);
-    const float su = DAG ? sp : sm, sd = DAG ? sm : sp;
-    Site<float, 1> o;
-    o.v[0] = fmaf(-0.5f, a0 + b0, fmaf(-su, DAG ? up.x : dn.x, diag * c.v[0]));
-    o.v[1] = fmaf(h, a0 - b0, fmaf(-sd, DAG ? dn.y : up.y, diag * c.v[1]));
-    o.v[2] = fmaf(-0.5f, a1 + b1, fmaf(-su, DAG ? up.z : dn.z, diag * c.v[2]));
-    o.v[3] = fmaf(h, a1 - b1, fmaf(-sd, DAG ? dn.w : up.w, diag * c.v[3]));
-    return o;
 }
 
 // dirac_combine's hop coefficients in float-float: P = -(r + 1) / 2,
@@ -2608,8 +2788,13 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
     // in shared memory): t64 is the output, so the last update's u survives
     // the reconstruction of chi
     double* const T = reinterpret_cast<double*>(S.xs32);
-    unsigned epoch = 0, gen = 0;
+    unsigned epoch = 0, gen = 0, sgen = 0;
+    bool slot_round = false;   // the last q pass ended in put_slots
     int staged_k = -1;
+    // The patch forms' cells are staged, and p formed, by every warp but the first,
+    // which the scalar step keeps (36 x 40 cells are three a thread either way)
+    constexpr int kIdle0 = PATCH ? 32 : 0, kStageNT = NT - kIdle0;
+    const int j0 = (int)threadIdx.x < kIdle0 ? NB : (int)threadIdx.x - kIdle0;
 #ifdef YK_CG_TIMING
     // block 0's cycles: reduce, A1 (with the staging wait), w/v/u, q, reliable
     // updates, round 0, the reconstruction of chi
@@ -2621,7 +2806,8 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
         const float* Rl = (mode == kRedo) ? S.r32[cur] : S.r32[prv];
         const float* Pl = S.p32[prv];
         const float* Al = prv == 0 ? S.Ap32 : S.t32;
-        for (int j = threadIdx.x; j < NB; j += NT) {
+#pragma unroll 1
+        for (int j = j0; j < NB; j += kStageNT) {
             const int m = buf_m(j);
             cp_async16(P_st + j, Pl + 4 * (size_t)m);
             cp_async16(R_st + j, Rl + 4 * (size_t)m);
@@ -2634,7 +2820,8 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
     auto pass_a1 = [&](int mode, int cur, int prv) {
         const SysLocal& L = sl[0];
         const W ar = L.f_alpha_re, beta = L.f_beta, cre = L.f_c_re, cim = L.f_c_im;
-        for (int j = threadIdx.x; j < NB; j += NT) {
+#pragma unroll 1
+        for (int j = j0; j < NB; j += kStageNT) {
             const int o = own_of(j);
             const bool is_own = o >= 0;
             const int m = is_own ? own_m(o) : 0;
@@ -2668,6 +2855,7 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
         Site<W, K> zero;
 #pragma unroll
         for (int i = 0; i < 4; ++i) zero.v[i] = W(0);
+#pragma unroll 1
         for (int j = SB + threadIdx.x; j < NB - SB; j += NT) {
             int t, b, du, dd;
             cell(j, 1, t, b, du, dd);
@@ -2679,6 +2867,7 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
             st_sm(Wp, j, h);
         }
         __syncthreads();
+#pragma unroll 1
         for (int j = 2 * SB + threadIdx.x; j < NB - 2 * SB; j += NT) {
             int t, b, du, dd;
             cell(j, 0, t, b, du, dd);
@@ -2689,6 +2878,7 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
             if (o >= 0) st_sm(V_own, o, v);
         }
         __syncthreads();
+#pragma unroll 1
         for (int j = 3 * SB + threadIdx.x; j < NB - 3 * SB; j += NT) {
             int t, b, du, dd;
             cell(j, 1, t, b, du, dd);
@@ -2705,6 +2895,35 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
     // Round 0 adds |eta|^2 of the compact index's two full sites in slot 5.
     auto pass_q = [&](int cur, bool round0) {
         float* Ac = cur == 0 ? S.Ap32 : S.t32;
+        if constexpr (PATCH) {
+            slot_round = s_fast && !round0;
+            if (slot_round) {
+                constexpr int OWN = kPT * kPX, T = (OWN + kTile - 1) / kTile, R = (T * kTile + NT - 1) / NT;
+                float f[4 * R];
+#pragma unroll
+                for (int i = 0; i < R; ++i) {
+                    const int o = threadIdx.x + i * NT;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) f[4 * i + c] = 0.f;
+                    if (o < OWN) {
+                        const int m = own_m(o), j = own_j(o);
+                        int t, b, du, dd;
+                        cell(j, 0, t, b, du, dd);
+                        const W sp = (t + 1 == Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
+                        const Site<W, K> v = ld_sm(Vp, j), r = ld_sm(R_st, j);
+                        const Site<W, K> q = eo_sm<true>(Wp, j, SB, du, dd, v, dep[j], rw, sp, sm);
+                        YK_ST(W, K, Ac, m, q);
+                        W dummy;
+                        f[4 * i] = site_norm2<W, K>(r);
+                        f[4 * i + 1] = site_norm2<W, K>(q);
+                        f[4 * i + 2] = site_norm2<W, K>(v);
+                        site_dot<W, K>(r, q, f[4 * i + 3], dummy);
+                    }
+                }
+                put_slots<T, R, NT>(a, tb, f, red, s_esc, ++epoch, sgen);
+                return;
+            }
+        }
         for (int base = tb; base < te; base += 2) {
             const int tile = base + hf;
             const bool tile_on = tile < te;
@@ -2745,14 +2964,21 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
     };
 
     auto reduce = [&](int kk, bool ru) -> bool {
-        auto prefetch = [&]() {
-            if (ru) return;
+        auto prefetch = [&](bool slots) -> int {
+            int bad = 0;
+            if (slots && threadIdx.x >= 32) {   // the staging warps' wait for the neighbours' q
+                const int d = threadIdx.x - 32;
+                if (d < deps.n) bad = wait_flag(a.flags + (size_t)deps.b[d] * kFlagStride, epoch, a.err);
+                asm volatile("bar.sync 1, %0;" ::"n"(NT - 32) : "memory");
+            }
+            if (ru) return bad;
             const int k1 = kk + 1;
             stage(kStep, k1 & 1, (k1 & 1) ^ 1);
             staged_k = k1;
+            return bad;
         };
-        return solo_reduce_body<K, true, true>(sa, gen, kk, ru, red, lst, sl[0], &s_nact, &s_anyru, s_cnt, s_esc, &s_fast, fsh,
-                                         prefetch);
+        return solo_reduce_body<K, true, true, PATCH>(sa, gen, kk, ru, red, lst, sl[0], &s_nact, &s_anyru, s_cnt,
+                                                               s_esc, &s_fast, fsh, sgen, slot_round && !ru, prefetch);
     };
 
     // the reliable update of iteration k, in float-float: fold chi_e += xs +
@@ -2885,7 +3111,7 @@ __global__ void __launch_bounds__(eo_threads(PX), PX == 8 ? 2 : 1) cg_eo_kernel(
         // bit; the own cells also go to rhs_e, r32[0] and p32[0].  Each thread
         // writes the cells that pass_a1 reads in the same thread.
         const HopFF hop = s_hop;
-        for (int j = threadIdx.x; j < NB; j += NT) {
+        for (int j = j0; j < NB; j += kStageNT) {
             const int m = buf_m(j);
             int t, b, du, dd;
             eo_geom(m, 0, Nh, sh, t, b, du, dd);
@@ -3632,7 +3858,10 @@ __global__ void __launch_bounds__(kHaloThreads) cg_eob_kernel(CGArgs a)
 // float-float as in the other even-odd kernels.  A patch is a chain of copies and
 // six passes with a barrier between them, so three 256-thread blocks share an SM,
 // each on a patch of its own (one 512-thread block, the next patch's copies in
-// flight: 91.7 ms for a step of 2 x 1024 x 1024, this 74.3).
+// flight: 91.7 ms for a step of 2 x 1024 x 1024, this 67.1; the
+// r = 1 form of 8 operations a spin pair was 4 ms slower, the passes being bound by
+// shared memory: six float4 a cell).  The two tiles' sums take one barrier and nine
+// shuffles (put_partial_ff for each: 66.7 ms, so 63.8).
 // ---------------------------------------------------------------------------
 constexpr int kEopPT = 32, kEopPX = 16, kEopSW = kEopPX + 4, kEopNB = kEopSW * (kEopPT + 8),
               kEopOwn = kEopPT * kEopPX;
@@ -3795,6 +4024,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
         const W rw = (W)S.r;
         const W ar = s_fa[P.q], beta = s_fb[P.q], cre = s_fc[P.q];
         // A1: p (and r on the own sites) on the buffer
+#pragma unroll 1
         for (int j = threadIdx.x; j < NB; j += NT) {
             const int o = own_of(j);
             const Site<W, K> po = ld_sm(P_st, j);
@@ -3823,10 +4053,11 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
 #pragma unroll
         for (int i = 0; i < 4; ++i) zero.v[i] = W(0);
         // w = -A_o^-1 H_oe p (odd) on [SB, NB - SB)
+#pragma unroll 1
         for (int j = SB + threadIdx.x; j < NB - SB; j += NT) {
             const int t = cell_t(P, j), b = (t + 1) & 1;
             const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
-            Site<W, K> h = eo_hop<false>(P_st, j, SB, b, zero, W(0), rw, sp, sm);
+            Site<W, K> h = eo_sm<false>(P_st, j, SB, b, b - 1, zero, W(0), rw, sp, sm);
             const W sc = -dip[j];
 #pragma unroll
             for (int i = 0; i < 4; ++i) h.v[i] *= sc;
@@ -3834,20 +4065,22 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
         }
         __syncthreads();
         // v = A_e p + H_eo w (even) on [2SB, NB - 2SB); the own sites' to v32
+#pragma unroll 1
         for (int j = 2 * SB + threadIdx.x; j < NB - 2 * SB; j += NT) {
             const int t = cell_t(P, j), b = t & 1;
             const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
-            const Site<W, K> v = eo_hop<false>(Wp, j, SB, b, ld_sm(P_st, j), dep[j], rw, sp, sm);
+            const Site<W, K> v = eo_sm<false>(Wp, j, SB, b, b - 1, ld_sm(P_st, j), dep[j], rw, sp, sm);
             st_sm(Vp, j, v);
             const int o = own_of(j);
             if (o >= 0) YK_ST(W, K, S.v32, own_m(P, o), v);
         }
         __syncthreads();
         // u = -A_o^-1 H^dag_oe v (odd) on [3SB, NB - 3SB)
+#pragma unroll 1
         for (int j = 3 * SB + threadIdx.x; j < NB - 3 * SB; j += NT) {
             const int t = cell_t(P, j), b = (t + 1) & 1;
             const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
-            Site<W, K> h = eo_hop<true>(Vp, j, SB, b, zero, W(0), rw, sp, sm);
+            Site<W, K> h = eo_sm<true>(Vp, j, SB, b, b - 1, zero, W(0), rw, sp, sm);
             const W sc = -dip[j];
 #pragma unroll
             for (int i = 0; i < 4; ++i) h.v[i] *= sc;
@@ -3856,7 +4089,10 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
         __syncthreads();
         // q = A_e v + H^dag_eo u on the own sites and the patch's partials
         // (round 0 adds |eta|^2 of the compact index's two full sites)
-        for (int hf = 0; hf < kEopOwn / kTile; ++hf) {
+        constexpr int T = kEopOwn / kTile;
+        float sums[4 * T];
+#pragma unroll
+        for (int hf = 0; hf < T; ++hf) {
             FF f[6];
 #pragma unroll
             for (int i = 0; i < 6; ++i) f[i] = FF{0.f, 0.f};
@@ -3866,7 +4102,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
                 const int t = cell_t(P, j), b = t & 1;
                 const W sp = (t + 1 == P.Nt) ? W(-1) : W(1), sm = (t == 0) ? W(-1) : W(1);
                 const Site<W, K> v = ld_sm(Vp, j);
-                const Site<W, K> qv = eo_hop<true>(Wp, j, SB, b, v, dep[j], rw, sp, sm);
+                const Site<W, K> qv = eo_sm<true>(Wp, j, SB, b, b - 1, v, dep[j], rw, sp, sm);
                 YK_ST(W, K, cur == 0 ? S.Ap32 : S.t32, m, qv);
                 const Site<W, K> r = ld_sm(R_st, j);
                 W rq, dummy;
@@ -3883,10 +4119,25 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
                 }
             }
             const int tile = s_t0[P.q] + 2 * P.lp + hf;
-            if (round0)
+            if (round0) {
                 put_partial_ff<(1 << 3), true>(a, tile, true, f, red);
-            else
-                put_partial_ff<kSkipIm, false>(a, tile, true, f, red);
+            } else {
+                sums[4 * hf] = f[0].hi;
+                sums[4 * hf + 1] = f[1].hi;
+                sums[4 * hf + 2] = f[2].hi;
+                sums[4 * hf + 3] = f[4].hi;
+            }
+        }
+        if (!round0) {
+            // (the last patch's warps have read s_w: its barriers lie between)
+            constexpr int hw = kTile / 32, rest = 32 / (4 * T);
+            static_assert(NT == kTile, "each tile's warps are the block's");
+            float* const s_w = reinterpret_cast<float*>(red);
+            const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+            const float v = warp_sums<4 * T>(sums);
+            if (lane % rest == 0) s_w[lane / rest * hw + w] = v;
+            __syncthreads();
+            if (w < 4) tile_partials<T>(a, s_t0[P.q] + 2 * P.lp, w, s_w);
         }
     };
 
@@ -4179,7 +4430,10 @@ __global__ void cg_prepare_kernel(CGArgs a)
         // generation 0: the coefficients of round 0 (never polled)
         for (int q = 0; q < 12; ++q) a.coef[i].w[q] = 0ull;
     }
-    for (int b = threadIdx.x; b < a.grid; b += blockDim.x) a.flags[(size_t)b * kFlagStride] = 0u;
+    for (int b = threadIdx.x; b < a.grid; b += blockDim.x) {
+        a.flags[(size_t)b * kFlagStride] = 0u;
+        for (int c = 0; c < 8; ++c) slot_word(a.flags, b, 0, 0)[c] = 0ull;
+    }
     if (threadIdx.x == 0) {
         *a.n_active = a.sys_count;
         *a.any_ru = 0;
