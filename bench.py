@@ -50,6 +50,7 @@ BYTES_CG_ITER_MIXED = 200          # unique bytes per site per FP32 CG iteration
 BYTES_CG_ITER_HALO = 128           # the same for cg_halo_kernel: D p stays in shared memory, diag is cached
 BYTES_CG_ITER_FP64 = 400
 BYTES_CG_ITER_EO = 48              # cg_eo_kernel: r, q, p loaded and stored per compact (even) site, 96 B = 48 B per site
+                                   # (cg_eoc_kernel keeps them on chip: the same work, no such traffic)
 # the thermalised start of the workload (both arms time the same steps from it)
 START = ROOT / "tests" / "golden" / "start_256x256.npz"
 DATA = ("synthetic: Philox noise; the timed steps continue a chain from tests/golden/start_256x256.npz, "
@@ -263,12 +264,12 @@ def roofline(pr, precision):
     """Roofline of the dominant kernel (the persistent CG) from the profiled
     steps: algorithmic bytes per launch / CUDA-event launch time."""
     per_launch_ms = pr.cg_ms / max(pr.cg_launches, 1)
-    halo, eo = pr.cg_kernel == 1, pr.cg_kernel == 3
+    halo, eo, clusters = pr.cg_kernel == 1, pr.cg_kernel == 3, pr.cg_kernel == 3 and pr.cg_grid <= 16
     if precision != "mixed":
         bpi = BYTES_CG_ITER_FP64
     else:
         bpi = BYTES_CG_ITER_EO if eo else (BYTES_CG_ITER_HALO if halo else BYTES_CG_ITER_MIXED)
-    kname = "cg_eo_kernel" if eo else ("cg_halo_kernel" if halo else
+    kname = "cg_eoc_kernel" if clusters else "cg_eo_kernel" if eo else ("cg_halo_kernel" if halo else
                                        f"cg_kernel<1,{'mixed' if precision == 'mixed' else 'fp64'}>")
     alg_bytes = pr.cg_site_iterations * bpi / max(pr.cg_launches, 1)
     pk = peaks()
@@ -277,9 +278,9 @@ def roofline(pr, precision):
     traffic = None
     if tr and tr.get("precision") == precision and tr.get("kernel", "cg_kernel<1,mixed>") == kname:
         traffic = tr["dram_bytes_per_iteration"] * pr.cg_iterations / max(pr.cg_launches, 1)
-    roof = {"bound": "hbm", "kernel": kname, "achieved": round(achieved, 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
+    roof = {"bound": "latency" if clusters else "hbm", "kernel": kname, "achieved": round(achieved, 1), "peak": pk["hbm_gbs"], "unit": "GB/s",
             "frac": round(achieved / pk["hbm_gbs"], 4), "traffic": traffic,
-            "peak_source": pk["source"], "bytes_per_site_iteration": bpi,
+            "peak_source": pk["source"], "bytes_per_site_iteration": bpi, "on_chip": clusters,
             "cg_iterations_per_step": pr.cg_iterations / max(pr.steps, 1),
             "ms_per_launch": round(per_launch_ms, 4), "profiled_steps": pr.steps}
     tot = pr.noise_ms + pr.cg_ms + pr.force_ms + pr.update_ms
@@ -415,10 +416,21 @@ def precision_errors(yk, torch, stream, phi_seg, step_seg, n, n_ops=5):
 # cg_eop_kernel: r, q, p, xs, v read and r, p, q, v, xs written per compact
 # site (w and u stay in shared memory; the halo re-reads are not counted):
 # 160 B, i.e. 80 B per lattice site.
+# cg_eoc_kernel (every lattice fits a cluster of 16 CTAs: 256 x 256 sites at most)
+# reports the code of the kernel it stands in for and keeps its vectors on chip;
+# its rate is counted at the 48 B of r, q and p.
 BATCHED_BYTES_PER_SITE_ITERATION = {4: 144, 5: 80}
 BATCHED_KERNELS = {0: "cg_kernel (grid-wide D^dag D)", 3: "cg_eo_kernel (single-system even-odd)",
                    4: "cg_eob_kernel (batched even-odd, four passes)",
                    5: "cg_eop_kernel (batched even-odd over 32 x 16 patches)"}
+
+
+def batched_kernel(pr, sites):
+    """Name and bytes per site and iteration of the batched step's CG on lattices of up to `sites` sites."""
+    if pr.cg_kernel in (4, 5) and sites <= 256 * 256 and not any(
+            os.environ.get(k) for k in ("YK_CG_EOC", "YK_CG_EO_PATCH", "YK_CG_EOP")):
+        return "cg_eoc_kernel (a cluster a system, even-odd)", BYTES_CG_ITER_EO
+    return BATCHED_KERNELS.get(pr.cg_kernel, str(pr.cg_kernel)), BATCHED_BYTES_PER_SITE_ITERATION.get(pr.cg_kernel, 144)
 
 
 def eob_roofline(yk, torch, stream, ctx):
@@ -430,9 +442,9 @@ def eob_roofline(yk, torch, stream, ctx):
         ctx.step(1)
     pr = ctx.profile_end()
     pk = peaks()
-    bps = BATCHED_BYTES_PER_SITE_ITERATION.get(pr.cg_kernel, 144)
+    name, bps = batched_kernel(pr, 1024 * 1024)
     gbs = pr.cg_site_iterations * bps / (pr.cg_ms / 1e3) / 1e9 if pr.cg_ms > 0 else 0.0
-    return {"kernel": BATCHED_KERNELS.get(pr.cg_kernel, str(pr.cg_kernel)), "cg_ms": round(pr.cg_ms, 3),
+    return {"kernel": name, "cg_ms": round(pr.cg_ms, 3),
             "bytes_per_site_iteration": bps, "achieved": round(gbs, 1), "unit": "GB/s",
             "peak": pk["hbm_gbs"], "frac": round(gbs / pk["hbm_gbs"], 4), "peak_source": pk["source"]}
 
@@ -552,16 +564,17 @@ def batched(yk, torch, stream, steps=20, warmup=3, n_chains=64, seed=1234):
     pr = ctx.profile_end()
     ctx.close()
     pk = peaks()
-    bps = BATCHED_BYTES_PER_SITE_ITERATION.get(pr.cg_kernel, 144)
+    name, bps = batched_kernel(pr, max(int(L) * int(L) for L in Ls))
     gbs = pr.cg_site_iterations * bps / (pr.cg_ms / 1e3) / 1e9 if pr.cg_ms > 0 else 0.0
     sites = int(sum(int(L) * int(L) for L in Ls))
     return {"config": f"{n_chains} chains, L in {{32,64,128,256}} (seed {seed}), 4 RHS, mixed CG rel-res 1e-10",
             "value": round(steps * n_chains / sec, 2), "unit": "chain-steps/s",
             "site_steps_per_s": round(steps * sites / sec, 1), "steps": steps,
             "ms_per_step": round(sec * 1e3 / steps, 3),
-            "cg_kernel": BATCHED_KERNELS.get(pr.cg_kernel, str(pr.cg_kernel)), "cg_grid": pr.cg_grid,
+            "cg_kernel": name, "cg_grid": pr.cg_grid,
             "cg_iterations_per_system_step": round(pr.cg_iterations / max(pr.steps * n_chains * 4, 1), 1),
-            "cg_roofline": {"bytes_per_site_iteration": bps, "achieved": round(gbs, 1),
+            "cg_roofline": {"bytes_per_site_iteration": bps, "on_chip": name.startswith("cg_eoc"),
+                            "achieved": round(gbs, 1),
                             "unit": "GB/s", "peak": pk["hbm_gbs"], "frac": round(gbs / pk["hbm_gbs"], 4)},
             "status_ok": all(o.status in (0, yk.YK_ENOCONV) for o in obs),
             "autotune": {"cg_grid": t.cg_grid, "cg_grid_max": t.cg_grid_max, "candidates": t.cg_candidates,

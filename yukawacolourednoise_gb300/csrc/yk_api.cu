@@ -968,11 +968,13 @@ int tune_overlap(yk_ctx* ctx)
 }
 
 // The autotuner.  Batched steps (several CG systems in one launch): the grid
-// of the persistent CG (the batched even-odd kernel's, or how many tiles
+// of the persistent CG (the batched even-odd kernels', or how many tiles
 // each block of cg_kernel owns), by timing the
 // step's CG (sources of Philox kind 100, which no step draws; 48 iterations;
 // two launches after one warm-up) at each candidate: the co-resident maximum,
-// 3/4 and 1/2 of it, one block per SM and half of that.  Fewer blocks own
+// 3/4 and 1/2 of it, one block per SM and half of that (the patch kernel: the
+// maximum, 2/3 of it and one block per SM); cluster solves of several forms: their
+// launches on parallel branches or one after another.  Fewer blocks own
 // more tiles each and synchronise fewer arrivals; more blocks hide latency.
 // The iterates do not depend on the grid (tile partials are summed in a fixed
 // order), so tuning never changes results.  The learned solver's convolution
