@@ -42,7 +42,6 @@ namespace {
 constexpr int kEcMaxC = 16;
 constexpr int kEcThreads = 512;
 constexpr int kEcMaxU = 4;
-constexpr long long kEcWaitCycles = 4000000000ll;   // about 2 s
 
 enum EcMode { kEcStep = 1, kEcRu = 2, kEcRedo = 3, kEcDone = 4 };
 
@@ -70,14 +69,7 @@ __device__ __forceinline__ float f4_dot(float4 a, float4 b, float s)
     return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, s))));
 }
 
-// Shared-memory address of this CTA's location `p` in CTA `rank`, and a store there.
-__device__ __forceinline__ unsigned cta_addr(const void* p, unsigned rank)
-{
-    unsigned q;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
-    return q;
-}
-
+// A store at such an address of another CTA.
 __device__ __forceinline__ void st_cta(unsigned addr, float4 v)
 {
     asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
@@ -113,49 +105,6 @@ __device__ __forceinline__ typename Part<R1>::T part_t(float4 s)
         return DAG == UP ? make_float2(s.x, s.z) : make_float2(s.y, s.w);
     else
         return s;
-}
-
-// Asynchronous stores into another CTA that count their bytes on its mbarrier.
-__device__ __forceinline__ void st_async(unsigned addr, float4 v, unsigned mbar)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
-                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(mbar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void st_async(unsigned addr, FF v, unsigned mbar)
-{
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(v.hi),
-                 "f"(v.lo), "r"(mbar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void mb_expect(unsigned mbar, unsigned bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
-}
-
-// Waits for the mbarrier's phase.  A wait that gives up (about 2 s) says so in
-// *dead, after which no wait of the CTA lasts and the solve ends.
-__device__ __forceinline__ void mb_wait(unsigned mbar, unsigned parity, int* dead)
-{
-    auto done = [&] {
-        unsigned ok;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(mbar), "r"(parity)
-                     : "memory");
-        return ok != 0;
-    };
-    if (done()) return;
-    const long long t0 = clock64();
-    while (!done())
-        if (*(volatile int*)dead || clock64() - t0 > kEcWaitCycles) {
-            *(volatile int*)dead = 1;
-            return;
-        }
 }
 
 // v, whose later uses the compiler does not merge with others

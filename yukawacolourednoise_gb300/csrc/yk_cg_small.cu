@@ -7,20 +7,21 @@
 // What bounds a small solve is latency: cg_kernel spends a neighbour sync, a grid
 // barrier and two round trips through L2 per iteration, and at FP64 (1/64 of the
 // FP32 rate on GB300) it forms r and p at five sites per site.  Microseconds an
-// iteration, cg_kernel and here: FP64 real 23.1 and 4.4 at 32 x 32, 23.3 and 8.5 at
-// 64 x 64, 23.5 and 19.9 at 128 x 96; FP64 complex 36.9 and 5.9 at 32 x 32; mixed
-// complex 12.4 and 3.7 at 64 x 64, 12.4 and 7.2 at 128 x 128.  Here a CTA owns a contiguous range of sites and keeps
+// iteration, cg_kernel and here: FP64 real 23.1 and 3.9 at 32 x 32, 23.3 and 8.1 at
+// 64 x 64, 23.5 and 19.5 at 128 x 96.  (With remote stores and two cluster barriers an
+// iteration: 4.4, 8.5 and 19.9; FP64 complex, 32 x 32: 36.9 and 5.9; mixed complex: 12.4
+// and 3.7 at 64 x 64, 12.4 and 7.2 at 128 x 128.)  Here a CTA owns a contiguous range of sites and keeps
 //   p, r, t = D_first p   in shared memory, on its sites and the Nx before and after,
 //   x (or the FP32 increment) and A p   of its own sites in registers,
-// and an iteration takes two cluster barriers:
+// and an iteration exchanges twice, by asynchronous stores counted on mbarriers:
 //   T: t = D_first p on the own sites; the edge sites' t is also stored into the
-//      neighbours' shared memory                                   -> barrier
+//      neighbours' shared memory                          -> neighbours
 //   B: A p = D_second t, its edges stored into the neighbours, the four sums'
-//      partials into every CTA of the cluster                      -> barrier
+//      partials into every CTA of the cluster             -> every CTA
 //   U: every CTA sums the partials in the same order and runs the same scalar
 //      step, then updates r and p on its own sites and, with the neighbours' A p,
 //      on the sites around them (redundantly: no third exchange).
-// All exchange is by remote stores before a barrier, all loads are local.
+// All exchange is by remote stores, all loads are local.
 //
 // A thread works on one flavour of a site (both spin entries, K planes): the
 // operator does not mix flavours (the pions' term reads the other one's entries).
@@ -122,7 +123,9 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
     using Un = Unit<W, K>;
     extern __shared__ __align__(16) unsigned char sm_raw[];
     __shared__ T wred[kSmThreads / 32][4];
-    __shared__ T cpart[kSmMaxC][4];
+    __shared__ __align__(8) T cpart[2][kSmMaxC][4];   // by the iteration's parity
+    __shared__ __align__(8) uint64_t mb[4];           // arrivals: t and A p around, cpart[0], cpart[1]
+    __shared__ int s_dead;                            // a wait gave up
     __shared__ SmState st;
     unsigned rank, nc;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -141,10 +144,9 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
     Un* const sa = stt + span;                       // A p on the sites around: before, after
     W* const sdiag = reinterpret_cast<W*>(sa + 4 * Nx);
     W* const spi = sdiag + omax;                     // g pi_a, when the chain carries pions
-    Un* const t_next = in_cta(stt, next);
-    Un* const t_prev = in_cta(stt, prev) + 2 * (Nx + prev_own);
-    Un* const a_next = in_cta(sa, next);
-    Un* const a_prev = in_cta(sa, prev) + 2 * Nx;
+    const unsigned t_next = cta_addr(stt, next), t_prev = cta_addr(stt + 2 * (Nx + prev_own), prev);
+    const unsigned a_next = cta_addr(sa, next), a_prev = cta_addr(sa + 2 * Nx, prev);
+    const unsigned mb0 = (unsigned)__cvta_generic_to_shared(mb), mb_next = cta_addr(mb, next), mb_prev = cta_addr(mb, prev);
     const bool first_dag = (a.mtype == YK_NORMAL);   // Normal: A = D D^dag, apply D^dag first
     const W s1st = first_dag ? W(-1) : W(1);
     const W r = (W)S.r;
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
         if constexpr (U >= 4) asm volatile("" ::: "memory");
     };
     // the four sums of the CTA's values into every CTA's cpart
-    auto partials = [&](const auto& v) {
+    auto partials = [&](const auto& v, int b, bool async) {
         const auto c = warp_sum4(v);
         if ((lane & 7) == 0) wred[warp][lane >> 3] = s_of(c, T{});
         __syncthreads();
@@ -233,14 +235,18 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
             t = s_add(t, s_shfl(t, 4));
             t = s_add(t, s_shfl(t, 2));
             t = s_add(t, s_shfl(t, 1));
-            for (unsigned c2 = w0; c2 < nc; c2 += 8) *in_cta(&cpart[rank][v4], c2) = t;
+            for (unsigned c2 = w0; c2 < nc; c2 += 8)
+                if (async)
+                    st_async(cta_addr(&cpart[b][rank][v4], c2), t, cta_addr(mb + 2 + b, c2));
+                else
+                    *in_cta(&cpart[b][rank][v4], c2) = t;
         }
     };
     // the cluster's sums, in every lane of warp 0
-    auto totals = [&](double (&s)[4]) {
+    auto totals = [&](double (&s)[4], int b) {
         const int v4 = lane >> 3, w0 = lane & 7;
-        T t = w0 < (int)nc ? cpart[w0][v4] : s_zero(T{});
-        if (w0 + 8 < (int)nc) t = s_add(t, cpart[w0 + 8][v4]);
+        T t = w0 < (int)nc ? cpart[b][w0][v4] : s_zero(T{});
+        if (w0 + 8 < (int)nc) t = s_add(t, cpart[b][w0 + 8][v4]);
         t = s_add(t, s_shfl(t, 4));
         t = s_add(t, s_shfl(t, 2));
         t = s_add(t, s_shfl(t, 1));
@@ -254,10 +260,24 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
         st.mode = kSmStep;
         st.iters = st.n_ru = st.status = st.converged = st.ru = 0;
         if (blockIdx.x == 0) *a.err = 0;
+        s_dead = 0;
+        for (int q = 0; q < 4; ++q)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb0 + 8u * q) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cluster_barrier();   // every CTA of the cluster has started: its shared memory can be written
 
+    // (How far apart CTAs can be: one sends the t of iteration k + 1 with every CTA's
+    // sums of iteration k, each sent after that CTA's last use of t_k, and A p of k + 1
+    // with the neighbours' t of k + 1, sent after they used A p of k; the sums
+    // alternate between two places.)
     for (int k = 0;; ++k) {
+        const int par = k & 1;
+        if (tid == 0) {
+            mb_expect(mb0, 4u * (unsigned)Nx * (unsigned)sizeof(Un));
+            mb_expect(mb0 + 8, 4u * (unsigned)Nx * (unsigned)sizeof(Un));
+            mb_expect(mb0 + 16 + 8 * par, 32u * nc);
+        }
         // ---------------- T
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -265,12 +285,13 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
             if (i < units) {
                 const Un t = apply(sp, u, s1st);
                 stt[i + 2 * Nx] = t;
-                if (i < 2 * Nx) t_prev[i] = t;
-                if (i >= units - 2 * Nx) t_next[i - (units - 2 * Nx)] = t;
+                if (i < 2 * Nx) st_async16(t_prev + (unsigned)(i * sizeof(Un)), t, mb_prev);
+                if (i >= units - 2 * Nx) st_async16(t_next + (unsigned)((i - (units - 2 * Nx)) * sizeof(Un)), t, mb_next);
             }
             unit_end();
         }
-        cluster_barrier();
+        __syncthreads();
+        mb_wait(mb0, par, &s_dead);
         // ---------------- B
         W v[4] = {W(0), W(0), W(0), W(0)};
 #pragma unroll
@@ -278,8 +299,8 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
             const int i = tid + u * TB;
             if (i < units) {
                 ap[u] = apply(stt, u, -s1st);
-                if (i < 2 * Nx) a_prev[i] = ap[u];
-                if (i >= units - 2 * Nx) a_next[i - (units - 2 * Nx)] = ap[u];
+                if (i < 2 * Nx) st_async16(a_prev + (unsigned)(i * sizeof(Un)), ap[u], mb_prev + 8);
+                if (i >= units - 2 * Nx) st_async16(a_next + (unsigned)((i - (units - 2 * Nx)) * sizeof(Un)), ap[u], mb_next + 8);
                 const Un rv = sr[i + 2 * Nx], pv = sp[i + 2 * Nx];
 #pragma unroll
                 for (int q = 0; q < 2 * K; ++q) {
@@ -291,13 +312,13 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
             }
             unit_end();
         }
-        partials(v);
-        cluster_barrier();
+        partials(v, par, true);
         // ---------------- the scalar step (scalar_step, yk_cg.cu; A is Hermitian, so
         // <p, A p> and alpha are real)
         if (warp == 0) {
+            mb_wait(mb0 + 16 + 8 * par, (k >> 1) & 1, &s_dead);
             double s[4];
-            totals(s);
+            totals(s, par);
             const double rr = s[0];
             SmState q = st;
             q.rr = rr;
@@ -317,7 +338,10 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
                 inv_rr = __shfl_sync(0xffffffffu, d, 1);
             }
             q.mode = kSmDone;
-            if (!isfinite(rr)) {
+            if (*(volatile int*)&s_dead) {
+                q.status = YK_ETIMEOUT;
+                if (lane == 0) *a.err = YK_ETIMEOUT;
+            } else if (!isfinite(rr)) {
                 q.status = YK_ENAN;
             } else if ((!MIXED || k == 0) && !(rr > q.stop2)) {
                 q.converged = 1;
@@ -347,6 +371,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
             if (lane == 0) st = q;
         }
         __syncthreads();
+        mb_wait(mb0 + 8, par, &s_dead);   // also at the end: nothing may come in after it
         if (st.mode == kSmDone) break;
         const W alpha = (W)st.alpha;
         W beta = (W)st.beta, cre = W(1), cim = W(0);
@@ -437,11 +462,11 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
                 T f4[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) f4[q] = s_of(w4[q], T{});
-                partials(f4);
+                partials(f4, par, false);
                 cluster_barrier();
                 if (warp == 0) {
                     double s[4];
-                    totals(s);
+                    totals(s, par);
                     SmState q = st;
                     const double rr = s[0];
                     q.rr = rr;

@@ -66,4 +66,74 @@ __device__ __forceinline__ T* in_cta(T* p, unsigned rank)
     return q;
 }
 
+constexpr long long kClusterWaitCycles = 4000000000ll;   // about 2 s
+
+// Shared-memory address of this CTA's location `p` in CTA `rank`.
+__device__ __forceinline__ unsigned cta_addr(const void* p, unsigned rank)
+{
+    unsigned q;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(q) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    return q;
+}
+
+// Asynchronous stores into another CTA that count their bytes on its mbarrier.
+__device__ __forceinline__ void st_async(unsigned addr, float4 v, unsigned mbar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(mbar)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_async(unsigned addr, FF v, unsigned mbar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr), "f"(v.hi),
+                 "f"(v.lo), "r"(mbar)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_async(unsigned addr, double v, unsigned mbar)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(__double_as_longlong(v)), "r"(mbar)
+                 : "memory");
+}
+
+// words of 16 bytes
+template <typename V>
+__device__ __forceinline__ void st_async16(unsigned addr, const V& v, unsigned mbar)
+{
+    static_assert(sizeof(V) % 16 == 0, "words of 16 bytes");
+    const float4* const p = reinterpret_cast<const float4*>(&v);
+#pragma unroll
+    for (int q = 0; q < (int)sizeof(V) / 16; ++q) st_async(addr + 16u * q, p[q], mbar);
+}
+
+__device__ __forceinline__ void mb_expect(unsigned mbar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+
+// Waits for the mbarrier's phase.  A wait that gives up (about 2 s) says so in
+// *dead, after which no wait of the CTA lasts and the solve ends.
+__device__ __forceinline__ void mb_wait(unsigned mbar, unsigned parity, int* dead)
+{
+    auto done = [&] {
+        unsigned ok;
+        asm volatile("{\n\t.reg .pred p;\n\t"
+                     "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok)
+                     : "r"(mbar), "r"(parity)
+                     : "memory");
+        return ok != 0;
+    };
+    if (done()) return;
+    const long long t0 = clock64();
+    while (!done())
+        if (*(volatile int*)dead || clock64() - t0 > kClusterWaitCycles) {
+            *(volatile int*)dead = 1;
+            return;
+        }
+}
+
 }  // namespace yk
