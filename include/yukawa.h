@@ -286,6 +286,11 @@ int yk_pcg_solve(yk_ctx* ctx, int chain, const double* b, double* x, double tol,
  * Returns YK_ETIMEOUT when the wait ran out as designed (the device stays
  * usable), YK_OK if it did not, YK_ECUDA on a CUDA error. */
 int yk_check_wait_timeout(void* stream, int* status);
+/* The same for a wait inside a cluster of four blocks, which all end together
+ * although the others pass more barriers than the one that gave up and store
+ * into its shared memory after that: YK_ETIMEOUT when every block learned of it
+ * and those stores arrived. */
+int yk_check_cluster_timeout(void* stream, int* status);
 
 /* FermionicDrift::getForce (code/src/FermionicDrift.cuh:15, FermionicDrift.cu:57-100):
  * F_n = -g Re sum_c conj(chi_{n,c}) eta_{n,c}, chi = D (D^dag D)^-1 eta, averaged

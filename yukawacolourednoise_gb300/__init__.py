@@ -168,6 +168,7 @@ _SIGS = {
                                      C.c_void_p, C.c_int, C.c_double, C.c_int, C.c_int, C.c_void_p,
                                      C.POINTER(SolveStats)]),
     "yk_check_wait_timeout": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
+    "yk_check_cluster_timeout": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     "yk_net_setup": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_uint64, C.c_double]),
     "yk_net_size": (C.c_int, [C.c_void_p, C.c_int]),
     "yk_net_weights": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_int]),

@@ -1789,11 +1789,11 @@ int yk_ctx_set_stream(yk_ctx* ctx, void* stream)
     return YK_OK;
 }
 
-int yk_check_wait_timeout(void* stream, int* status)
+static int check_timeout(int (*probe)(cudaStream_t, int*), const char* name, void* stream, int* status)
 {
     int st = 0;
-    if (wait_timeout_probe(static_cast<cudaStream_t>(stream), &st) != 0) {
-        set_error("yk_check_wait_timeout: %s", cudaGetErrorString(cudaGetLastError()));
+    if (probe(static_cast<cudaStream_t>(stream), &st) != 0) {
+        set_error("%s: %s", name, cudaGetErrorString(cudaGetLastError()));
         return YK_ECUDA;
     }
     if (status) *status = st;
@@ -1802,6 +1802,16 @@ int yk_check_wait_timeout(void* stream, int* status)
         return YK_ETIMEOUT;
     }
     return YK_OK;
+}
+
+int yk_check_wait_timeout(void* stream, int* status)
+{
+    return check_timeout(wait_timeout_probe, "yk_check_wait_timeout", stream, status);
+}
+
+int yk_check_cluster_timeout(void* stream, int* status)
+{
+    return check_timeout(cluster_timeout_probe, "yk_check_cluster_timeout", stream, status);
 }
 
 int yk_ctx_synchronize(yk_ctx* ctx)

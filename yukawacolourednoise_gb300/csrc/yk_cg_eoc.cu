@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kEcThreads, 1) cg_eoc_kernel(CGArgs a, const i
     __shared__ FF wred[kEcThreads / 32][4];
     __shared__ __align__(8) FF cpart[2][kEcMaxC][4];   // by the iteration's parity
     __shared__ __align__(8) uint64_t mb[4];   // arrivals: VH, QH, cpart[0], cpart[1]
-    __shared__ int s_dead;
+    __shared__ int s_dead, s_left;
     __shared__ EcState st;
     __shared__ SysDev S;     // the compact view
     __shared__ EcView g;
@@ -407,7 +407,7 @@ __global__ void __launch_bounds__(kEcThreads, 1) cg_eoc_kernel(CGArgs a, const i
         if (tid < n) reinterpret_cast<uint64_t*>(&S)[tid] = reinterpret_cast<const uint64_t*>(a.sys + sys)[tid];
         if (tid == 0) {
             st.iters = sys;   // for the end: where the state goes
-            s_dead = 0;
+            s_dead = s_left = 0;
             for (int q = 0; q < 4; ++q)
                 asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(mb + q)));
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -874,7 +874,11 @@ __global__ void __launch_bounds__(kEcThreads, 1) cg_eoc_kernel(CGArgs a, const i
         o.mode = 0;
         o.chi_ready = 2;   // however the solve ended
     }
-    cluster_barrier();   // no CTA leaves while another may still store into it
+    if (cluster_end(nc, &s_dead, &s_left, a.err) && rank == 0 && tid == 0) {
+        CGState& o = *out_state;
+        o.converged = 0;
+        o.status = YK_ETIMEOUT;
+    }
 }
 
 // ---------------------------------------------------------------------------

@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
     __shared__ T wred[kSmThreads / 32][4];
     __shared__ __align__(8) T cpart[2][kSmMaxC][4];   // by the iteration's parity
     __shared__ __align__(8) uint64_t mb[4];           // arrivals: t and A p around, cpart[0], cpart[1]
-    __shared__ int s_dead;                            // a wait gave up
+    __shared__ int s_dead, s_left;                    // a wait gave up; CTAs that then came to the end
     __shared__ SmState st;
     unsigned rank, nc;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
         st.mode = kSmStep;
         st.iters = st.n_ru = st.status = st.converged = st.ru = 0;
         if (blockIdx.x == 0) *a.err = 0;
-        s_dead = 0;
+        s_dead = s_left = 0;
         for (int q = 0; q < 4; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb0 + 8u * q) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -575,7 +575,53 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
         o.mode = 0;
         o.chi_ready = st.ru;   // an update has just left D_first x of this x in t64
     }
-    cluster_barrier();   // no CTA leaves while another may still store into it
+    if (cluster_end(nc, &s_dead, &s_left, a.err) && rank == 0 && tid == 0) {
+        CGState& o = a.st[sys];
+        o.converged = 0;
+        o.status = YK_ETIMEOUT;
+    }
+}
+
+// Failure detection without a fault: four CTAs, of which CTA 1 waits for bytes that nobody
+// sends, gives up and ends, while the others pass two more barriers, as in a reliable
+// update, and then store into it.  out: the stores that CTA 1 found when all had
+// come to the end, and the CTAs that learned of the timeout.
+constexpr int kProbeCtas = 4;
+__device__ int g_cluster_probe[3];   // err, out[2]
+
+__global__ void __launch_bounds__(64) cluster_timeout_probe_kernel(int* err, int* out)
+{
+    __shared__ __align__(8) uint64_t mb[2];
+    __shared__ __align__(8) double in[kProbeCtas];
+    __shared__ int s_dead, s_left;
+    unsigned rank;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const unsigned mb0 = (unsigned)__cvta_generic_to_shared(mb);
+    if (threadIdx.x == 0) {
+        s_dead = s_left = 0;
+        for (int q = 0; q < kProbeCtas; ++q) in[q] = 0.0;
+        for (int q = 0; q < 2; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb0 + 8u * q) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        mb_expect(mb0, 16u);   // never sent
+        mb_expect(mb0 + 8u, 8u * (kProbeCtas - 1));
+    }
+    __syncthreads();
+    cluster_barrier();
+    if (rank == 1) {
+        mb_wait(mb0, 0, &s_dead);
+    } else {
+        cluster_barrier();
+        cluster_barrier();
+        if (threadIdx.x == 0) st_async(cta_addr(&in[rank], 1), 1.0, cta_addr(mb + 1, 1));
+    }
+    const bool late = cluster_end(kProbeCtas, &s_dead, &s_left, err);
+    if (threadIdx.x == 0) {
+        if (late) atomicAdd(out + 1, 1);
+        if (rank == 1) {
+            mb_wait(mb0 + 8u, 0, &s_dead);
+            out[0] = (int)(in[0] + in[2] + in[3]);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -711,6 +757,34 @@ cudaError_t launch_cg_small(const CGArgs& a, int K, bool mixed, const OneLattice
     int pions = lat.pions;
     void* args[] = {&b, &pions};
     return cudaLaunchKernelExC(&cfg, small_fn(K, mixed, f.u), args);
+}
+
+int cluster_timeout_probe(cudaStream_t stream, int* status)
+{
+    void* p = nullptr;
+    int h[3] = {};
+    cudaError_t e = cudaGetSymbolAddress(&p, g_cluster_probe);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, sizeof(h), stream);
+    if (e == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(kProbeCtas);
+        cfg.blockDim = dim3(64);
+        cfg.stream = stream;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = kProbeCtas;
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int *err = (int*)p, *out = err + 1;
+        void* args[] = {&err, &out};
+        e = cudaLaunchKernelExC(&cfg, (const void*)cluster_timeout_probe_kernel, args);
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, p, sizeof(h), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e != cudaSuccess) return -1;
+    *status = h[1] == kProbeCtas - 1 && h[2] == kProbeCtas ? h[0] : 0;
+    return 0;
 }
 
 }  // namespace yk

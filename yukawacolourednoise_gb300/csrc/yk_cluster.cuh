@@ -136,4 +136,31 @@ __device__ __forceinline__ void mb_wait(unsigned mbar, unsigned parity, int* dea
         }
 }
 
+// The end of a solve: no CTA leaves while another may still store into it.  After a
+// wait that gave up the CTAs no longer pass the same barriers (the one that gave up ends,
+// the others may still be in a reliable update), so it tells every CTA, which ends its
+// waits too, and those that know arrive at barriers until all have come here (*left
+// counts them in each), then let the stores on their way arrive.  A CTA that gave up comes here
+// with no more barriers behind it than any CTA's last one, so nobody leaves uninformed.
+// Returns whether a wait gave up, and says so in *err.
+__device__ __forceinline__ bool cluster_end(unsigned nc, int* dead, int* left, int* err)
+{
+    const unsigned tid = threadIdx.x;
+    if (__syncthreads_or(*(volatile int*)dead) && tid < nc) *(volatile int*)in_cta(dead, tid) = 1;
+    cluster_barrier();
+    if (!*(volatile int*)dead) return false;
+    if (tid < nc) atomicAdd(in_cta(left, tid), 1);
+    const long long t0 = clock64();
+    int more = 1;
+    while (more) {
+        cluster_barrier();
+        more = __syncthreads_or(tid == 0 && *(volatile int*)left < (int)nc && clock64() - t0 < 4 * kClusterWaitCycles);
+    }
+    const long long t1 = clock64();
+    while (clock64() - t1 < 200000) {
+    }
+    if (tid == 0) *err = YK_ETIMEOUT;
+    return true;
+}
+
 }  // namespace yk

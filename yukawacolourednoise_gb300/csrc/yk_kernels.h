@@ -56,6 +56,8 @@ void cg_halo_init();
 // Runs the wait-timeout probe kernel on `stream`; *status = the device status
 // it recorded.  Returns 0, or -1 on a CUDA error.
 int wait_timeout_probe(cudaStream_t stream, int* status);
+// The same for the waits inside a cluster (yk_cg_small.cu).
+int cluster_timeout_probe(cudaStream_t stream, int* status);
 
 // Cluster-resident mixed CG (yk_cg_cluster.cu): one 16-CTA cluster per system
 // of real (K = 1) vectors whose rows fit the cluster (cg_cluster_fits);
