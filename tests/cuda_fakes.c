@@ -1,0 +1,36 @@
+/* Preloaded before libyukawa_gb300.so in a child process: calls of the CUDA
+ * runtime that do more, or less, than they are asked to. */
+#define _GNU_SOURCE
+#include <cuda_runtime_api.h>
+#include <dlfcn.h>
+
+static void *real(const char *name)
+{
+    return dlsym(dlopen("libcudart.so.13", RTLD_LAZY | RTLD_NOLOAD), name);
+}
+
+static void *word;   /* the context's error word: what it last read as four bytes */
+static int launches_to_go, status;
+
+/* Before the n-th cluster or cooperative launch from now on the error word becomes
+ * `st`, as if a wait of the kernel before it had given up. */
+void fake_error(int n, int st)
+{
+    launches_to_go = n;
+    status = st;
+}
+
+cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, enum cudaMemcpyKind kind, cudaStream_t s)
+{
+    cudaError_t (*f)(void *, const void *, size_t, enum cudaMemcpyKind, cudaStream_t) = real("cudaMemcpyAsync");
+    if (n == 4 && kind == cudaMemcpyDeviceToHost) word = (void *)src;
+    return f(dst, src, n, kind, s);
+}
+
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *cfg, const void *fn, void **args)
+{
+    cudaError_t (*f)(const cudaLaunchConfig_t *, const void *, void **) = real("cudaLaunchKernelExC");
+    if (launches_to_go > 0 && --launches_to_go == 0)
+        cudaMemcpyAsync(word, &status, 4, cudaMemcpyHostToDevice, cfg->stream);
+    return f(cfg, fn, args);
+}

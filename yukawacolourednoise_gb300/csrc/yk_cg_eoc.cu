@@ -296,12 +296,15 @@ __device__ __noinline__ float4 ec_update(const EcView& g, float al, bool only_od
 // chi_e = 0, rhs_e = eta_e - H^dag_eo A_o^-1 eta_o, and the tile's |eta|^2
 // (its partial's first slot).  A kernel of its own because it has the whole GPU:
 // inside the solve it took 26 of 195 us at 256 x 256, on 16 SMs.  A block forms
-// -A_o^-1 eta_o on its tile and a row around it in shared memory.
+// -A_o^-1 eta_o on its tile and a row around it in shared memory.  err, when given, is
+// cleared: here, before all solves of the step, since one that starts late would clear
+// what another has recorded.
 template <bool R1>
-__global__ void __launch_bounds__(kTile) eoc_prepare_kernel(CGArgs a)
+__global__ void __launch_bounds__(kTile) eoc_prepare_kernel(CGArgs a, int* err)
 {
     extern __shared__ __align__(16) float4 ep_raw[];   // high parts, then low
     __shared__ FF red[kTile / 32];
+    if (err && blockIdx.x == 0 && threadIdx.x == 0) *err = 0;
     const int idx = a.tile_begin + (int)blockIdx.x;
     const int2 tl = a.eo_tiles[idx];
     const SysDev& S = a.sys[tl.x];         // the compact view
@@ -638,7 +641,6 @@ __global__ void __launch_bounds__(kEcThreads, 1) cg_eoc_kernel(CGArgs a, const i
             del[h] = e.lo;
         }
     }
-    if (tid == 0 && blockIdx.x == 0) *a.err = 0;
     cluster_barrier();   // every CTA of the cluster has started: its shared memory can be written
     diagonals();
 #pragma unroll
@@ -1127,13 +1129,14 @@ static CGArgs eoc_args(const CGArgs& a)
     return b;
 }
 
-cudaError_t launch_eoc_prepare(const CGArgs& a, bool r1, bool other, int max_nh, cudaStream_t stream)
+cudaError_t launch_eoc_prepare(const CGArgs& a, bool r1, bool other, int max_nh, cudaStream_t stream, bool first)
 {
     const CGArgs b = eoc_args(a);
     const int n = a.tile_end - a.tile_begin;
     const size_t smem = 2 * sizeof(float4) * (kTile + 2 * (size_t)max_nh);
-    if (r1) eoc_prepare_kernel<true><<<n, kTile, smem, stream>>>(b);
-    if (other) eoc_prepare_kernel<false><<<n, kTile, smem, stream>>>(b);
+    int* const err = first ? b.err : nullptr;
+    if (r1) eoc_prepare_kernel<true><<<n, kTile, smem, stream>>>(b, err);
+    if (other) eoc_prepare_kernel<false><<<n, kTile, smem, stream>>>(b, err);
     return cudaGetLastError();
 }
 
@@ -1175,7 +1178,7 @@ cudaError_t launch_plane_solve(const CGArgs& a0, const EocForm& f, const double*
     for (int stage = 0; stage < 2; ++stage) {
         a.st = a0.st + 2 * stage;
         a.stop2 = stop2 + 2 * stage;
-        cudaError_t e = launch_eoc_prepare(a, f.r1, !f.r1, f.nh, stream);
+        cudaError_t e = launch_eoc_prepare(a, f.r1, !f.r1, f.nh, stream, stage == 0);
         if (e == cudaSuccess) e = launch_cg_eoc(a, f, nullptr, 2, stream);
         if (e != cudaSuccess) return e;
         if (stage == 0) plane_mid_kernel<<<dim3(blocks, 2), kBlock, 0, stream>>>(a.sys, a.sys_eo, normal ? -1 : 1);

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kSmThreads, 1) cg_small_kernel(CGArgs a, int p
         st.c_re = 1.0;
         st.mode = kSmStep;
         st.iters = st.n_ru = st.status = st.converged = st.ru = 0;
-        if (blockIdx.x == 0) *a.err = 0;
+        if (blockIdx.x == 0) *a.err = 0;   // (the solve's one launch: another CTA's wait gives up 2 s later)
         s_dead = s_left = 0;
         for (int q = 0; q < 4; ++q)
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mb0 + 8u * q) : "memory");

@@ -33,10 +33,11 @@ void cg_small_init();
 // to `spread` times the fewest CTAs; the launch for `count` systems of one form,
 // order[0 .. count) or, order null, from a.sys_first on (a as for launch_cg with
 // its compact views given); before it what the solves of a's tiles start from, for
-// systems of r = 1 and others, the widest of max_nh columns; the kernels' attributes (before any capture).
+// systems of r = 1 and others, the widest of max_nh columns (first: no solve since the error
+// word was last read, which is then cleared); the kernels' attributes (before any capture).
 bool cg_eoc_form(int Nt, int Nh, double r, int spread, EocForm* f);
 cudaError_t launch_cg_eoc(const CGArgs& a, const EocForm& f, const int* order, int count, cudaStream_t stream);
-cudaError_t launch_eoc_prepare(const CGArgs& a, bool r1, bool other, int max_nh, cudaStream_t stream);
+cudaError_t launch_eoc_prepare(const CGArgs& a, bool r1, bool other, int max_nh, cudaStream_t stream, bool first = true);
 void cg_eoc_init();
 // A x = b for a complex source by two such solves of its planes (yk_cg_eoc.cu).
 size_t plane_norm_doubles();
