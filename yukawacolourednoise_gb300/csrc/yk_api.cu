@@ -789,7 +789,7 @@ int ws_solve(yk_ctx* ctx, int c, int count, int mtype, double tol, int tol_mode,
     EocForm form;
     const char* eo = getenv("YK_CG_EO");
     if (count == 1 && precision == YK_MIXED && !C.pions && !beside && C.Nt % 2 == 0 && C.Nx % 2 == 0 && C.Nx >= 4 &&
-        !(eo && eo[0] == '0') && cg_eoc_form(C.Nt, C.Nx / 2, C.a.r, kEocSpread, &form)) {
+        !(tol_mode == YK_TOL_REL && plane_out_of_reach(tol, C.a.r)) && !(eo && eo[0] == '0') && cg_eoc_form(C.Nt, C.Nx / 2, C.a.r, kEocSpread, &form)) {
         bool done = false;
         if (int rc = plane_solve(ctx, c, form, mtype, tol, tol_mode, max_iter, stats, &done)) return rc;
         if (done) return YK_OK;

@@ -41,6 +41,7 @@ cudaError_t launch_eoc_prepare(const CGArgs& a, bool r1, bool other, int max_nh,
 void cg_eoc_init();
 // A x = b for a complex source by two such solves of its planes (yk_cg_eoc.cu).
 size_t plane_norm_doubles();
+bool plane_out_of_reach(double tol, double r);   // a relative target that such solves cannot meet
 cudaError_t launch_plane_solve(const CGArgs& a, const EocForm& f, const double* b, double* x, const double* sigma, int Nt,
                                int Nx, double m0, double g, double r, double* norm, double* resid, double* stop2,
                                double* tmp, cudaStream_t stream);
