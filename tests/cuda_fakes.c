@@ -20,6 +20,17 @@ void fake_error(int n, int st)
     status = st;
 }
 
+static int no_memory;
+
+/* From now on (on) every device allocation fails, or none does (off). */
+void fake_no_memory(int on) { no_memory = on; }
+
+cudaError_t cudaMalloc(void **p, size_t n)
+{
+    cudaError_t (*f)(void **, size_t) = real("cudaMalloc");
+    return no_memory ? cudaErrorMemoryAllocation : f(p, n);
+}
+
 cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, enum cudaMemcpyKind kind, cudaStream_t s)
 {
     cudaError_t (*f)(void *, const void *, size_t, enum cudaMemcpyKind, cudaStream_t) = real("cudaMemcpyAsync");

@@ -88,3 +88,19 @@ with yk.Context(params(64)) as ctx:
     st = ctx.cg_solve(buffer(b), buffer(b), tol=1e-10, tol_mode=yk.YK_TOL_REL, max_iter=5000, precision=yk.YK_MIXED)
     assert st.converged == 1
 """)
+
+
+def test_no_memory_for_the_planes(child):
+    # a mixed solve that finds no room for the plane solves' workspace runs on the one there
+    # is; with room again it takes the planes
+    child("""
+b, x = (buffer(np.random.default_rng(1).normal(size=(64 * 64, 8))) for _ in range(2))
+solve = dict(tol=1e-10, tol_mode=yk.YK_TOL_REL, max_iter=5000)
+with yk.Context(params(64)) as ctx:
+    ctx.cg_solve(b, x, precision=yk.YK_FP64, **solve)   # the workspace of every solve
+    fakes.fake_no_memory(1)
+    st = ctx.cg_solve(b, x, precision=yk.YK_MIXED, **solve)
+    assert st.converged == 1
+    fakes.fake_no_memory(0)
+    assert ctx.cg_solve(b, x, precision=yk.YK_MIXED, **solve).reliable_updates > st.reliable_updates   # two solves' updates
+""")

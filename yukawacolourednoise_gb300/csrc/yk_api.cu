@@ -728,14 +728,14 @@ int ensure_planes(yk_ctx* ctx, int c)
 }
 
 // A mixed solve of one complex source on a lattice that cg_eoc_kernel takes.
-// *done false: it did not reach the target on the FP64 residual (or within
-// max_iter), and the caller solves otherwise.
+// *done false: there is no memory for the planes, or it did not reach the target on
+// the FP64 residual (or within max_iter), and the caller solves otherwise.
 int plane_solve(yk_ctx* ctx, int c, const EocForm& form, int mtype, double tol, int tol_mode, int max_iter,
                 yk_solve_stats* stats, bool* done)
 {
     Chain& C = ctx->ch[c];
     *done = false;
-    if (int rc = ensure_planes(ctx, c)) return rc;
+    if (int rc = ensure_planes(ctx, c)) return rc == YK_ENOMEM ? YK_OK : rc;
     const PlaneWs& w = *C.planes;
     const SysDev& S = C.ws.h_sys[0];
     CGArgs a = base_args(ctx);
