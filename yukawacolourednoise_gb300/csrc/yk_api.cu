@@ -221,6 +221,7 @@ struct yk_ctx {
     // the step's solves by cg_eoc_kernel (empty: not taken): groups of systems of
     // one form, their systems in d_eoc_order, launched on parallel branches
     // (eoc_parallel; else one after another: the autotuner's choice)
+    bool eoc_wanted = true;    // YK_CG_EO=0, YK_CG_EOC=0 and others at context creation: no such solves
     std::vector<EocGroup> eoc;
     int* d_eoc_order = nullptr;
     bool eoc_parallel = true;
@@ -787,9 +788,9 @@ int ws_solve(yk_ctx* ctx, int c, int count, int mtype, double tol, int tol_mode,
     Chain& C = ctx->ch[c];
     Workspace& w = C.ws;
     EocForm form;
-    const char* eo = getenv("YK_CG_EO");
-    if (count == 1 && precision == YK_MIXED && !C.pions && !beside && C.Nt % 2 == 0 && C.Nx % 2 == 0 && C.Nx >= 4 &&
-        !(tol_mode == YK_TOL_REL && plane_out_of_reach(tol, C.a.r)) && !(eo && eo[0] == '0') && cg_eoc_form(C.Nt, C.Nx / 2, C.a.r, kEocSpread, &form)) {
+    if (ctx->eoc_wanted && count == 1 && precision == YK_MIXED && !C.pions && !beside && C.Nt % 2 == 0 && C.Nx % 2 == 0 &&
+        C.Nx >= 4 && !(tol_mode == YK_TOL_REL && plane_out_of_reach(tol, C.a.r)) &&
+        cg_eoc_form(C.Nt, C.Nx / 2, C.a.r, kEocSpread, &form)) {
         bool done = false;
         if (int rc = plane_solve(ctx, c, form, mtype, tol, tol_mode, max_iter, stats, &done)) return rc;
         if (done) return YK_OK;
@@ -1169,12 +1170,9 @@ int pion_setup(yk_ctx* ctx)
 // SMs at once (kEocCtas: eight GPCs' clusters of 16): a lone small system is
 // bound by the latency of a CTA's passes, a batch by its SMs' throughput, where
 // the fewest CTAs a system (the least work on edge rows) is best.
-// YK_CG_EOC=0, or YK_CG_EO_PATCH / YK_CG_EOP, which choose among the other
-// even-odd kernels, turn this off.
 int eoc_setup(yk_ctx* ctx, const std::vector<SysDev>& views)
 {
-    const char* env = getenv("YK_CG_EOC");
-    if ((env && env[0] == '0') || getenv("YK_CG_EO_PATCH") || getenv("YK_CG_EOP")) return YK_OK;
+    if (!ctx->eoc_wanted) return YK_OK;
     std::vector<EocForm> form(views.size());
     for (int spread = kEocSpread;; spread /= 2) {
         int ctas = 0;
@@ -1422,6 +1420,11 @@ int yk_ctx_create(const yk_params* params, int n_chains, yk_ctx** out)
         }
         ctx->cg_cluster = want && cg_cluster_init();
         ctx->cluster_sites = sites;
+        // solves by cg_eoc_kernel, of the step and of complex sources: YK_CG_EO_PATCH and
+        // YK_CG_EOP choose among the other even-odd kernels
+        const char* oe = getenv("YK_CG_EO");
+        const char* ce = getenv("YK_CG_EOC");
+        ctx->eoc_wanted = !(oe && oe[0] == '0') && !(ce && ce[0] == '0') && !getenv("YK_CG_EO_PATCH") && !getenv("YK_CG_EOP");
         const char* he = getenv("YK_CG_HALO");
         ctx->cg_halo = !(he && he[0] == '0');
         const char* ne = getenv("YK_NOISE_OVERLAP");
