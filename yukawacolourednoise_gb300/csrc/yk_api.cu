@@ -414,10 +414,15 @@ CGArgs step_cg_args(yk_ctx* ctx)
     return a;
 }
 
-// The one lattice of every system of the step (Nt 0: they differ).
+// Whether the step's batched solves take block ranges balanced by the previous step's iterations.
+bool step_balanced(const yk_ctx* ctx) { return ctx->nsys > 1 && ctx->cg_balance && !ctx->cg_eo; }
+
+// The one lattice of every system of the step (Nt 0: they differ, or their block
+// ranges are balanced, which only the grid-wide kernel does).
 OneLattice step_lattice(const yk_ctx* ctx)
 {
     OneLattice q = {};
+    if (step_balanced(ctx)) return q;
     for (const Chain& C : ctx->ch) {
         if (C.n_rhs_step == 0) continue;
         if (q.Nt && (q.Nt != C.Nt || q.Nx != C.Nx)) return {};
@@ -519,7 +524,7 @@ int enqueue_step(yk_ctx* ctx)
             prof_end(ctx, 1, e, (int)ctx->eoc.size() + 1);
         } else {
             // batched: block ranges balanced by the previous step's iterations
-            const bool bal = ctx->nsys > 1 && ctx->cg_balance && !ctx->cg_eo;
+            const bool bal = step_balanced(ctx);
             if (bal) a.balance = ctx->d_balance;
             YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, &ctx->cg_grid, &ctx->cg_kernel,
                             step_lattice(ctx)));
@@ -1020,7 +1025,8 @@ int run_autotune(yk_ctx* ctx)
         T.cg_grid = T.cg_grid_max = step_cg_grid(ctx);
         T.cg_ms_chosen = std::min(ms[0], ms[1]);
         T.cg_ms_max = std::max(ms[0], ms[1]);
-    } else if (ctx->nsys > 1 && !ctx->cg_cluster && ctx->eoc.empty()) {
+    } else if (ctx->nsys > 1 && !ctx->cg_cluster && ctx->eoc.empty() &&
+               !cg_small_grid(step_cg_args(ctx), 1, mixed, step_lattice(ctx))) {   // whose clusters have no grid to choose
         const int maxg = !ctx->cg_eo ? cg_max_grid(1, mixed)
                        : ctx->eo_patches ? cg_eop_max_grid(ctx->nsys) : cg_eob_max_grid();
         // the patch kernel's blocks are a third of an SM's: fewer than one an SM is never
