@@ -1007,7 +1007,10 @@ int run_autotune(yk_ctx* ctx)
             rc = prepare_step_eoc(ctx, a);
             if (rc == YK_OK) rc = launch_step_eoc(ctx, a);
             if (rc == YK_OK) e = cudaEventRecord(e0, ctx->stream);
-            for (int rep = 0; rep < 2 && rc == YK_OK && e == cudaSuccess; ++rep) rc = launch_step_eoc(ctx, a);
+            for (int rep = 0; rep < 2 && rc == YK_OK && e == cudaSuccess; ++rep) {
+                rc = prepare_step_eoc(ctx, a);   // a solve starts from what the last one changed
+                if (rc == YK_OK) rc = launch_step_eoc(ctx, a);
+            }
             if (rc == YK_OK && e == cudaSuccess) e = cudaEventRecord(e1, ctx->stream);
             if (rc == YK_OK && e == cudaSuccess) e = cudaEventSynchronize(e1);
             if (rc == YK_OK && e == cudaSuccess) e = cudaEventElapsedTime(&ms[cand], e0, e1);
