@@ -38,8 +38,21 @@ cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, enum cudaMemcp
     return f(dst, src, n, kind, s);
 }
 
+static int launches;
+
+/* Kernels launched until now. */
+int fake_launches(void) { return launches; }
+
+cudaError_t __cudaLaunchKernel(void *k, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t s)
+{
+    cudaError_t (*f)(void *, dim3, dim3, void **, size_t, cudaStream_t) = real("__cudaLaunchKernel");
+    ++launches;
+    return f(k, grid, block, args, smem, s);
+}
+
 cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *cfg, const void *fn, void **args)
 {
+    ++launches;
     cudaError_t (*f)(const cudaLaunchConfig_t *, const void *, void **) = real("cudaLaunchKernelExC");
     if (launches_to_go > 0 && --launches_to_go == 0)
         cudaMemcpyAsync(word, &status, 4, cudaMemcpyHostToDevice, cfg->stream);

@@ -104,3 +104,18 @@ with yk.Context(params(64)) as ctx:
     fakes.fake_no_memory(0)
     assert ctx.cg_solve(b, x, precision=yk.YK_MIXED, **solve).reliable_updates > st.reliable_updates   # two solves' updates
 """)
+
+
+@pytest.mark.parametrize("chains", ["params(32), params(64, wilson_param=0.7)", "params(32, precision=yk.YK_FP64)",
+                                    "params(128, precision=yk.YK_FP64)", "params(64, cut_fraction=0.35)", "params(512)",
+                                    "params(33), params(20)"])
+def test_launches_of_a_profiled_step(child, chains):
+    child(f"""
+with yk.Context([{chains}]) as ctx:
+    ctx.step(1)
+    ctx.profile_begin()
+    n = fakes.fake_launches()
+    ctx.step(2)
+    n = fakes.fake_launches() - n
+    assert ctx.profile_end().launches == n, n
+""")

@@ -432,8 +432,8 @@ OneLattice step_lattice(const yk_ctx* ctx)
     return q;
 }
 
-// What the step's solves by cg_eoc_kernel start from.
-int prepare_step_eoc(yk_ctx* ctx, const CGArgs& a)
+// What the step's solves by cg_eoc_kernel start from.  launched (may be null): the kernels it took.
+int prepare_step_eoc(yk_ctx* ctx, const CGArgs& a, int* launched = nullptr)
 {
     bool r1 = false, other = false;
     int nh = 0;
@@ -442,6 +442,7 @@ int prepare_step_eoc(yk_ctx* ctx, const CGArgs& a)
         nh = std::max(nh, G.form.nh);
     }
     YK_CK(launch_eoc_prepare(a, r1, other, nh, ctx->stream));
+    if (launched) *launched = (r1 ? 1 : 0) + (other ? 1 : 0);
     return YK_OK;
 }
 
@@ -511,7 +512,8 @@ int enqueue_step(yk_ctx* ctx)
             ctx->cg_kernel = 2;
             prof_end(ctx, 1, e, 2);
         } else if (!ctx->eoc.empty()) {
-            if (int rc = prepare_step_eoc(ctx, a)) return rc;
+            int prepared = 0;
+            if (int rc = prepare_step_eoc(ctx, a, &prepared)) return rc;
             if (overlap) YK_CK(cudaEventRecord(ctx->fork_ev, ctx->stream));
             if (int rc = launch_step_eoc(ctx, a)) return rc;
             // the noise after the clusters in the order of the launches: its blocks
@@ -521,7 +523,7 @@ int enqueue_step(yk_ctx* ctx)
                 if (int rc = beside()) return rc;
             ctx->cg_grid = step_cg_grid(ctx);
             ctx->cg_kernel = ctx->nsys == 1 ? 3 : ctx->eo_patches ? 5 : 4;
-            prof_end(ctx, 1, e, (int)ctx->eoc.size() + 1);
+            prof_end(ctx, 1, e, (int)ctx->eoc.size() + prepared);
         } else {
             // batched: block ranges balanced by the previous step's iterations
             const bool bal = step_balanced(ctx);
@@ -529,7 +531,7 @@ int enqueue_step(yk_ctx* ctx)
             YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, &ctx->cg_grid, &ctx->cg_kernel,
                             step_lattice(ctx)));
             if (bal) YK_CK(launch_cg_balance(a, ctx->cg_grid, ctx->d_balance, ctx->stream));
-            prof_end(ctx, 1, e, bal ? 3 : 2);
+            prof_end(ctx, 1, e, bal ? 3 : ctx->cg_kernel == 6 ? 1 : 2);   // (cg_small_kernel prepares itself)
         }
     }
     StepArgs s = step_args(ctx);
