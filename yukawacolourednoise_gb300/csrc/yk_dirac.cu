@@ -175,7 +175,13 @@ __global__ void __launch_bounds__(kBlock) dirac_kernel(const R* __restrict__ in,
         R diag;
         if constexpr (sizeof(R) == 4) {
             const FF sf = ff_split(sg), q = ff_add(df, ff_mul(gf, sf));
-            diag = isfinite(q.hi) ? q.hi : fmaf(gf.hi, sf.hi, df.hi);
+            diag = q.hi;
+            // a field value or a coupling beyond FP32's range, in FP64 (asm: the compiler would
+            // do so always and select)
+            if (!isfinite(q.hi) || (sf.hi == 0.f && __double2hiint(sg) << 1 != 0))
+                asm volatile("{\n\t.reg .f64 d;\n\tfma.rn.f64 d, %1, %2, %3;\n\tcvt.rn.f32.f64 %0, d;\n\t}"
+                             : "=f"(diag)
+                             : "d"(g), "d"(sg), "d"(diag0));
         } else {
             diag = fma(g, sg, diag0);
         }
@@ -234,9 +240,10 @@ static cudaError_t launch_t(const void* in, void* out, const double* sigma, cons
     const int gx = (Nx + kBlock - 1) / kBlock;
     int band = (int)((int64_t)gx * Nt / (4 * 152));
     band = band < 1 ? 1 : band > 4 ? 4 : band;
-    // g and the diagonal's constant as float-float, by the host
+    // g and the diagonal's constant as float-float, by the host (NaN for a g that FP32 holds
+    // with fewer bits or not at all: the kernel takes FP64 then)
     const double diag0 = 2.0 * r + m0;
-    const float gh = (float)g, dh = (float)diag0;
+    const float gh = g == 0.0 || (fabs(g) > 0x1p-100 && fabs(g) < 0x1p100) ? (float)g : NAN, dh = (float)diag0;
     const float4 ff = make_float4(gh, (float)(g - gh), dh, (float)(diag0 - dh));
     dirac_kernel<R, K, DAG, R1><<<gx * ((Nt + band - 1) / band), kBlock, 0, stream>>>(
         (const R*)in, (R*)out, sigma, pi, Nt, Nx, gx, band, diag0, g, r, ff);
