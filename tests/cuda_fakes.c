@@ -38,6 +38,33 @@ cudaError_t cudaMemcpyAsync(void *dst, const void *src, size_t n, enum cudaMemcp
     return f(dst, src, n, kind, s);
 }
 
+static int device, cluster_attributes;
+
+/* From now on the current device calls itself `d`. */
+void fake_device(int d) { device = d; }
+
+cudaError_t cudaGetDevice(int *d)
+{
+    *d = device;
+    return cudaSuccess;
+}
+
+cudaError_t cudaDeviceGetAttribute(int *v, enum cudaDeviceAttr a, int d)
+{
+    cudaError_t (*f)(int *, enum cudaDeviceAttr, int) = real("cudaDeviceGetAttribute");
+    return f(v, a, d == device ? 0 : d);
+}
+
+/* Kernels opted in to clusters of more than eight blocks until now. */
+int fake_cluster_attributes(void) { return cluster_attributes; }
+
+cudaError_t cudaFuncSetAttribute(const void *fn, enum cudaFuncAttribute a, int v)
+{
+    cudaError_t (*f)(const void *, enum cudaFuncAttribute, int) = real("cudaFuncSetAttribute");
+    cluster_attributes += a == cudaFuncAttributeNonPortableClusterSizeAllowed;
+    return f(fn, a, v);
+}
+
 static int launches;
 
 /* Kernels launched until now. */

@@ -119,3 +119,21 @@ with yk.Context([{chains}]) as ctx:
     n = fakes.fake_launches() - n
     assert ctx.profile_end().launches == n, n
 """)
+
+
+def test_cluster_kernels_on_another_device(child):
+    # kernel attributes hold for one device: a process that makes contexts on two sets them for
+    # both (here one device that calls itself another)
+    child("""
+def attributes():
+    n = fakes.fake_cluster_attributes()
+    with yk.Context(params(32, precision=yk.YK_FP64)) as ctx:
+        ctx.step(1)
+        assert ctx.observables().status == 0
+    return fakes.fake_cluster_attributes() - n
+
+first = attributes()
+assert first > 0 and attributes() == 0
+fakes.fake_device(1)
+assert attributes() == first
+""")

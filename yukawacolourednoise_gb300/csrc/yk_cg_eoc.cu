@@ -1084,7 +1084,7 @@ const void* eoc_fn(const EocForm& f)
 // that can be resident (16, or 8 where a GPC holds no 16; 0: none).
 int eoc_max_cluster()
 {
-    static const int most = [] {
+    return once_per_device([] {
         int best = kEcMaxC;
         for (int q = 0; q <= 2 * kEcMaxU; ++q) {
             const void* fn = eoc_fn({1, 1 + q / 2, 0, 0, q < 2 * kEcMaxU, q % 2 != 0});
@@ -1117,8 +1117,7 @@ int eoc_max_cluster()
             }
         }
         return best;
-    }();
-    return most;
+    });
 }
 
 // The form of a lattice on clusters of c CTAs.

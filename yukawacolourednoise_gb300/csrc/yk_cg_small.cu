@@ -655,7 +655,7 @@ const void* small_fn(int K, bool mixed, int u)
 // cluster that can be resident (16, or 8 where a GPC holds no 16).
 int small_max_cluster()
 {
-    static const int most = [] {
+    return once_per_device([] {
         int best = 0;
         for (int K = 1; K <= 2; ++K)
             for (int m = 0; m <= (K == 2 ? 1 : 0); ++m)
@@ -691,8 +691,7 @@ int small_max_cluster()
                     }
                 }
         return best;
-    }();
-    return most;
+    });
 }
 
 }  // namespace

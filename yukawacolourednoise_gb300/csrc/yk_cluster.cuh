@@ -2,9 +2,25 @@
 // run inside one thread-block cluster (yk_cg_small.cu, yk_cg_eoc.cu).
 #pragma once
 
+#include <mutex>
+
 #include "yk_ff.cuh"
 
 namespace yk {
+
+// f() once for each device of the process: a kernel's attributes hold for the device that
+// was current.
+template <typename F>
+int once_per_device(F f)
+{
+    constexpr int kDevices = 64;
+    static std::once_flag once[kDevices];
+    static int value[kDevices];
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return f();
+    std::call_once(once[dev], [&] { value[dev] = f(); });
+    return value[dev];
+}
 
 // A sum in the precision it is carried: FP64, or float-float for FP32 vectors.
 __device__ __forceinline__ double s_add(double a, double b) { return a + b; }
