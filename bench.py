@@ -264,7 +264,7 @@ def roofline(pr, precision):
     """Roofline of the dominant kernel (the persistent CG) from the profiled
     steps: algorithmic bytes per launch / CUDA-event launch time."""
     per_launch_ms = pr.cg_ms / max(pr.cg_launches, 1)
-    halo, eo, clusters = pr.cg_kernel == 1, pr.cg_kernel == 3, pr.cg_kernel == 3 and pr.cg_grid <= 16
+    halo, eo, clusters = pr.cg_kernel == 1, pr.cg_kernel == 3, pr.cg_kernel == 3 and pr.cg_cluster_blocks > 0
     if precision != "mixed":
         bpi = BYTES_CG_ITER_FP64
     else:
@@ -425,10 +425,9 @@ BATCHED_KERNELS = {0: "cg_kernel (grid-wide D^dag D)", 3: "cg_eo_kernel (single-
                    5: "cg_eop_kernel (batched even-odd over 32 x 16 patches)"}
 
 
-def batched_kernel(pr, sites):
-    """Name and bytes per site and iteration of the batched step's CG on lattices of up to `sites` sites."""
-    if pr.cg_kernel in (4, 5) and sites <= 256 * 256 and not any(
-            os.environ.get(k) for k in ("YK_CG_EOC", "YK_CG_EO_PATCH", "YK_CG_EOP")):
+def batched_kernel(pr):
+    """Name and bytes per site and iteration of the batched step's CG."""
+    if pr.cg_kernel in (4, 5) and pr.cg_cluster_blocks > 0:
         return "cg_eoc_kernel (a cluster a system, even-odd)", BYTES_CG_ITER_EO
     return BATCHED_KERNELS.get(pr.cg_kernel, str(pr.cg_kernel)), BATCHED_BYTES_PER_SITE_ITERATION.get(pr.cg_kernel, 144)
 
@@ -442,7 +441,7 @@ def eob_roofline(yk, torch, stream, ctx):
         ctx.step(1)
     pr = ctx.profile_end()
     pk = peaks()
-    name, bps = batched_kernel(pr, 1024 * 1024)
+    name, bps = batched_kernel(pr)
     gbs = pr.cg_site_iterations * bps / (pr.cg_ms / 1e3) / 1e9 if pr.cg_ms > 0 else 0.0
     return {"kernel": name, "cg_ms": round(pr.cg_ms, 3),
             "bytes_per_site_iteration": bps, "achieved": round(gbs, 1), "unit": "GB/s",
@@ -564,7 +563,7 @@ def batched(yk, torch, stream, steps=20, warmup=3, n_chains=64, seed=1234):
     pr = ctx.profile_end()
     ctx.close()
     pk = peaks()
-    name, bps = batched_kernel(pr, max(int(L) * int(L) for L in Ls))
+    name, bps = batched_kernel(pr)
     gbs = pr.cg_site_iterations * bps / (pr.cg_ms / 1e3) / 1e9 if pr.cg_ms > 0 else 0.0
     sites = int(sum(int(L) * int(L) for L in Ls))
     return {"config": f"{n_chains} chains, L in {{32,64,128,256}} (seed {seed}), 4 RHS, mixed CG rel-res 1e-10",

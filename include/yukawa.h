@@ -388,6 +388,8 @@ typedef struct yk_profile {
                                  /*   on a cluster per system where all fit one   */
                                  /*   (cg_grid: the clusters' blocks), else on    */
                                  /*   the whole GPU                               */
+    int cg_cluster_blocks;       /* blocks of the largest cluster that solved one */
+                                 /*   system (kernels 3 to 6; 0: the whole GPU)   */
     double noise_ms, cg_ms, force_ms, update_ms;   /* summed device time          */
     int64_t cg_iterations;       /* CG iterations, summed over systems            */
     int64_t cg_site_iterations;  /* sum over chains of iterations x volume        */

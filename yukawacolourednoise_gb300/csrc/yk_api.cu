@@ -175,6 +175,7 @@ struct yk_ctx {
     bool io_kernel = true;
     int cg_grid = 0;
     int cg_kernel = 0;   // kernel of the last step CG launch (yk_profile.cg_kernel)
+    int cg_cluster_blocks = 0;   // of the largest of its clusters, where a system has one
     // mixed precision with every step system fitting one 16-CTA cluster and
     // YK_CG_CLUSTER=1 in the environment: the cluster-resident CG instead of
     // the grid-wide kernel
@@ -523,6 +524,7 @@ int enqueue_step(yk_ctx* ctx)
                 if (int rc = beside()) return rc;
             ctx->cg_grid = step_cg_grid(ctx);
             ctx->cg_kernel = ctx->nsys == 1 ? 3 : ctx->eo_patches ? 5 : 4;
+            ctx->cg_cluster_blocks = ctx->eoc[0].form.c;   // the largest first
             prof_end(ctx, 1, e, (int)ctx->eoc.size() + prepared);
         } else {
             // batched: block ranges balanced by the previous step's iterations
@@ -531,6 +533,7 @@ int enqueue_step(yk_ctx* ctx)
             YK_CK(launch_cg(a, 1, ctx->precision == YK_MIXED, ctx->stream, &ctx->cg_grid, &ctx->cg_kernel,
                             step_lattice(ctx)));
             if (bal) YK_CK(launch_cg_balance(a, ctx->cg_grid, ctx->d_balance, ctx->stream));
+            ctx->cg_cluster_blocks = ctx->cg_kernel == 6 ? ctx->cg_grid / ctx->nsys : 0;
             prof_end(ctx, 1, e, bal ? 3 : ctx->cg_kernel == 6 ? 1 : 2);   // (cg_small_kernel prepares itself)
         }
     }
@@ -2328,6 +2331,7 @@ int yk_profile_end(yk_ctx* ctx, yk_profile* out)
     }
     out->cg_grid = ctx->cg_grid;
     out->cg_kernel = ctx->cg_kernel;
+    out->cg_cluster_blocks = ctx->cg_cluster_blocks;
     ctx->profiling = false;
     return YK_OK;
 }
