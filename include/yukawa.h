@@ -100,7 +100,9 @@ typedef struct yk_action {
 } yk_action;
 
 typedef struct yk_solve_stats {
-    int iterations;            /* CG iterations (summed over right-hand sides)   */
+    int iterations;            /* CG iterations (summed over right-hand sides; of */
+                               /*   a mixed complex source by its planes the sum */
+                               /*   of two even-odd solves', at half the work)   */
     int reliable_updates;      /* FP64 residual recomputations (mixed)           */
     double rr;                 /* final |r|^2 of the solver                      */
     double rr0;                /* |b|^2                                          */
@@ -191,7 +193,11 @@ int yk_dirac_apply(yk_ctx* ctx, int chain, const void* in, void* out, int dagger
  * CGsolver.cu:42-59): solve A x = b with A = D^dag D (YK_DAGGER) or D D^dag
  * (YK_NORMAL), x0 = 0.  b and x are FP64 complex.  precision YK_FP64 runs the
  * reference's plain CG; YK_MIXED runs FP32 iterations with FP64 reliable
- * updates and an FP64 final residual check.  Returns YK_ENOCONV if the cap
+ * updates and an FP64 final residual check.  On even lattices that fit a
+ * cluster (256 x 256 and smaller) a mixed solve takes two even-odd solves of
+ * b's real and imaginary planes, whose updates are in float-float (48 bits):
+ * the result stands if its FP64 residual meets the target, else, and for
+ * targets below 2^-46 |b| / (about) 3 |D|, the other solve runs.  Returns YK_ENOCONV if the cap
  * is hit (the reference stops silently, CGsolver.cu:107). */
 int yk_cg_solve(yk_ctx* ctx, int chain, const void* b, void* x, int mtype, double tol,
                 int tol_mode, int max_iter, int precision, yk_solve_stats* stats);
@@ -325,7 +331,10 @@ int yk_langevin_step_io(yk_ctx* ctx, int chain, const double* phi_in, double* ph
  * fixed, main.cu:258-266).  Batched contexts (several CG systems per step):
  * the grid of the step's persistent CG, i.e. how many 256-site tiles each
  * block owns, chosen by timing the step's CG at candidate grids (the
- * co-resident maximum, 3/4 and 1/2 of it, one block per SM, half of that).
+ * co-resident maximum, 3/4 and 1/2 of it, one block per SM, half of that; of
+ * the patch kernel the maximum, 2/3 of it and one block per SM).  Clusters have
+ * no such grid: where a batch's even-odd clusters are of several forms, whether
+ * these run side by side or one after another is timed.
  * Where the step's coloured noise and the next step's sources run -- on an
  * auxiliary stream beside the CG, on the SMs the CG's grid leaves free, or on
  * the main stream after the CG -- is chosen by timing whole steps of both forms

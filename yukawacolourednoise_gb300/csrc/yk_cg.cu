@@ -3858,9 +3858,9 @@ __global__ void __launch_bounds__(kHaloThreads) cg_eob_kernel(CGArgs a)
 // float-float as in the other even-odd kernels.  A patch is a chain of copies and
 // six passes with a barrier between them, so three 256-thread blocks share an SM,
 // each on a patch of its own (one 512-thread block, the next patch's copies in
-// flight: 91.7 ms for a step of 2 x 1024 x 1024, this 67.1; the
-// r = 1 form of 8 operations a spin pair was 4 ms slower, the passes being bound by
-// shared memory: six float4 a cell).  The two tiles' sums take one barrier and nine
+// flight: 91.7 ms for a step of 2 x 1024 x 1024, this 67.1; with the r = 1 form of 8
+// operations a spin pair 71.5: fewer operations do not help, nor did fewer loads from
+// shared memory by strips of four rows, so that a patch's chain of copies and barriers is left).  The two tiles' sums take one barrier and nine
 // shuffles (put_partial_ff for each: 66.7 ms, so 63.8).
 // ---------------------------------------------------------------------------
 constexpr int kEopPT = 32, kEopPX = 16, kEopSW = kEopPX + 4, kEopNB = kEopSW * (kEopPT + 8),
@@ -4174,7 +4174,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
         }
     };
 
-    // Runs f(S, q, m, tile, tile_on, on) for every site of this block's share
+    // Runs f(S, q, m, tile, on) for every site of this block's share
     // of the tiles of the systems in `mask`.
     auto for_sites = [&](int mask, auto&& f) {
         eob_scan<NT>(nsys, s_mode, s_nt, mask, s_pre);
@@ -4182,13 +4182,12 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
         eob_share(s_pre[nsys], &lo, &hi);
         int qc = -1;
         for (int ii = lo; ii < hi; ++ii) {
-            const bool tile_on = true;
             const int q = (qc >= 0 && ii >= s_pre[qc] && ii < s_pre[qc + 1]) ? qc : eob_find(ii, nsys, s_pre);
             qc = q;
             const int lt = ii - s_pre[q];
             const SysDev& S = a.sys[a.sys_first + q];
             const int m = lt * kTile + ts;
-            f(S, q, m, s_t0[q] + lt, tile_on, tile_on && m < S.V);
+            f(S, q, m, s_t0[q] + lt, m < S.V);
         }
     };
     struct Geo {
@@ -4209,7 +4208,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
 
     // ---------------- round 0: eta of both classes (b, full layout), A_e and
     // 1 / A_o, -A_o^-1 eta_o (t64), chi_e = xs = v = 0; then rhs_e, r_0 = p_0
-    for_sites(kAll, [&](const SysDev& S, int q, int m, int, bool, bool on) {
+    for_sites(kAll, [&](const SysDev& S, int q, int m, int, bool on) {
         if (!on) return;
         const SysDev& SF = a.sys_full[a.sys_first + q];
         const int Ve = S.V;
@@ -4246,7 +4245,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
         YK_ST(W, K, S.v32, m, zw);
     });
     if (!eob_barrier(a, gen)) return;
-    for_sites(kAll, [&](const SysDev& S, int q, int m, int, bool, bool on) {
+    for_sites(kAll, [&](const SysDev& S, int q, int m, int, bool on) {
         if (!on) return;
         const SysDev& SF = a.sys_full[a.sys_first + q];
         const Geo g = geo(S, m, 0);
@@ -4274,7 +4273,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
         if (nact == 0) break;
         pass(false);
         // kRu: fold chi_e += xs + alpha v (float-float); xs = 0
-        for_sites(1 << kRu, [&](const SysDev& S, int q, int m, int, bool, bool on) {
+        for_sites(1 << kRu, [&](const SysDev& S, int q, int m, int, bool on) {
             if (!on) return;
             SiteFF xv = ld_ff(S.x, m);
             const Site<W, K> xs = YK_LD(W, K, S.xs32, m);
@@ -4292,7 +4291,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
             YK_ST(W, K, S.xs32, m, zw);
         });
         // kRu2: u = -A_o^-1 H^dag_oe chi_e (odd, t64)
-        for_sites(1 << kRu2, [&](const SysDev& S, int, int m, int, bool, bool on) {
+        for_sites(1 << kRu2, [&](const SysDev& S, int, int m, int, bool on) {
             if (!on) return;
             const Geo g = geo(S, m, 1);
             SiteFF zero;
@@ -4305,7 +4304,7 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
             st_ff(S.t64, m, h);
         });
         // kRu3: r = rhs_e - (A_e chi_e + H^dag_eo u); |r|^2, <r, p_{k-1}>
-        for_sites(1 << kRu3, [&](const SysDev& S, int q, int m, int tile, bool tile_on, bool on) {
+        for_sites(1 << kRu3, [&](const SysDev& S, int q, int m, int tile, bool on) {
             const int cur = s_par[q], prv = cur ^ 1;
             float v0 = 0.f, v2 = 0.f;
             if (on) {
@@ -4329,14 +4328,14 @@ __global__ void __launch_bounds__(kEopThreads, 3) cg_eop_kernel(CGArgs a)
             for (int i = 0; i < 6; ++i) f[i] = FF{0.f, 0.f};
             f[0] = FF{v0, 0.f};
             f[2] = FF{v2, 0.f};
-            put_partial_ff<(1 << 1) | (1 << 4) | (1 << 5) | kSkipIm, true>(a, tile, tile_on, f, red);
+            put_partial_ff<(1 << 1) | (1 << 4) | (1 << 5) | kSkipIm, true>(a, tile, true, f, red);
         });
         if (!eop_reduce(a, gen, k, red, &s_active, &s_ru, s_mode, s_par)) return;
         ++k;
     }
     // chi of both classes in the full layout (t64) for the force
     if (!eob_barrier(a, gen)) return;
-    for_sites(kAll | (1 << kIdle), [&](const SysDev& S, int q, int m, int, bool, bool on) {
+    for_sites(kAll | (1 << kIdle), [&](const SysDev& S, int q, int m, int, bool on) {
         if (!on) return;
         const SysDev& SF = a.sys_full[a.sys_first + q];
         Geo g = geo(S, m, 0);
@@ -4745,12 +4744,12 @@ static cudaError_t launch_cg_t(const CGArgs& a0, cudaStream_t stream, int* grid_
                                           : (const void*)cg_eo_kernel<0>;
                 return cudaLaunchKernelExC(&cfg, fn, args);
             }
-            // lattices that 16 x 16 patches tile: the batched patch kernel
-            // (YK_CG_EOP=0: the four-pass kernel below), one block per SM
+            // lattices that 32 x 16 patches tile: the batched patch kernel
+            // (YK_CG_EOP=0: the four-pass kernel below), up to three blocks an SM
             const char* pe = getenv("YK_CG_EOP");
             if (a.eo_patches && !(pe && pe[0] == '0') && eop_max_grid(a.sys_count) > 0) {
                 int pg = capped(eop_max_grid(a.sys_count), a.grid_cap);
-                const int want = a.eo_tile_end - a.eo_tile_begin;   // patches (one tile each)
+                const int want = a.eo_tile_end - a.eo_tile_begin;   // tiles, two a patch
                 if (pg > want) pg = want;
                 if (pg < 1) pg = 1;
                 e.grid = pg;

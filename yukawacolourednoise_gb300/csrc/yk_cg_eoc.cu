@@ -11,12 +11,14 @@
 // sums leaves it in an iteration:
 //   w = -A_o^-1 H_oe p      on the own rows and one around them
 //   v = A_e p + H_eo w      on the own rows; its edge rows also go into the
-//                           neighbours' shared memory       -> cluster barrier
+//                           neighbours' shared memory       -> their threads at the edges
 //   u = -A_o^-1 H^dag_oe v  on the own rows and one around them
-//   q = A_e v + H^dag_eo u  on the own rows; edge rows and the sums' partials
-//                           into the other CTAs             -> cluster barrier
+//   q = A_e v + H^dag_eo u  on the own rows; edge rows into the neighbours, the
+//                           sums' partials into every CTA   -> the scalar step, then q's rows
 //   chi_e += alpha v, r -= alpha q, p = r + beta p on the own rows; r and p also
 //                           on the two rows around them, from the neighbours' q
+// What leaves is stored asynchronously and counted on the receiver's mbarriers, and only those
+// threads wait that read it; there is no cluster barrier but in an update.
 // Systems run independently: no block waits for another system's.
 //
 // A thread owns up to U consecutive rows of one compact column, and the chi

@@ -42,7 +42,7 @@ namespace {
 constexpr int kSmMaxC = 16;
 constexpr int kSmThreads = 512;
 constexpr size_t kSmMaxSmem = 220 * 1024;
-constexpr int kSmMaxReal = 12288;   // sites of a real FP64 solve
+constexpr int kSmMaxReal = 12288;   // sites of a real FP64 solve (small_form)
 
 // FP64 data of global memory that another CTA of the cluster wrote before the
 // last barrier: served by L2.
@@ -698,10 +698,12 @@ int small_max_cluster()
 
 // Whether the solve's systems, all on one lattice, take cg_small_kernel: its
 // CTAs per system, threads and units a thread.  A real FP64 solve stays in the
-// cluster up to 12288 sites: there the 16 SMs' FP64 pipes need as long as
-// cg_kernel's synchronisations over the whole GPU (128 x 96: 19.9 against 23.5 us
-// an iteration; 128 x 128: 25.6 against 23.6).  Complex solves stay while their
-// vectors fit.
+// cluster up to 12288 sites (128 x 96: 19.5 us an iteration here, 23.5 in cg_kernel).
+// The 16 SMs' FP64 pipes need as long as cg_kernel's synchronisations over the whole
+// GPU a little above that: 112 x 112 20.7 against 23.8 us, 120 x 120 22.9 against 23.9,
+// 128 x 128 25.3 against 23.7 (the line was drawn before the exchange by mbarriers; of
+// several systems each has its own SMs here: four of 128 x 128 25.3 against 39.7).
+// Complex solves stay while their vectors fit.
 static bool small_form(const CGArgs& a, int K, bool mixed, const OneLattice& lat, SmForm* f)
 {
     const int Nt = lat.Nt, Nx = lat.Nx;
@@ -717,7 +719,11 @@ static bool small_form(const CGArgs& a, int K, bool mixed, const OneLattice& lat
         return u <= (mixed ? 6 : 4) && small_smem(V, Nx, q, K, mixed, lat.pions != 0) <= kSmMaxSmem;
     };
     if (!fits(c)) return false;
-    // 32 sites a CTA at least, and no more CTAs than the GPU holds at once
+    // 32 sites a CTA at least, and up to 288 CTAs in all: 18 clusters of 16, as many as are
+    // resident at two such CTAs an SM (us an iteration, 32 x 32, 18 systems on 16 CTAs each
+    // 6.4, on 8 7.6; 36 on 8 7.9, on 16 12.2; 64 x 64, 18 on 16 24.0, on 8 27.1).  It is not
+    // the best for every count: 54 x 45, 24 systems on 8 18.1, on 4 16.1; 32 x 32, 19 on 8
+    // 7.6, on 16 6.5.
     while (c > 1 && (V / c < 32 || (long long)c * a.sys_count > 288) && fits(c / 2)) c /= 2;
     const int units = 2 * ((V + c - 1) / c);
     int u = 1;

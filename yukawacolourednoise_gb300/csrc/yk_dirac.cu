@@ -10,12 +10,12 @@
 // the diagonal and adds the hops in three grid-synced passes).  Complex (K = 2)
 // applies add the pion term g i gamma5 tau.pi when the chain carries pions.
 //
-// FP32 is bound by HBM (2048 x 2048: 51 us, 5.9 TB/s; its diagonal in float-float
+// FP32 is bound by HBM (2048 x 2048: 43.9 us, 6.9 TB/s; its diagonal in float-float
 // on the FP32 pipes), FP64 by its pipe, 1/64 of the FP32 rate: at r = 1 a time hop
 // keeps one spin entry and an x hop a combination u -+ d, so that a spin pair and
-// plane takes 8 operations against 14 (1000 x 749: 58 us against 87, of which
+// plane takes 8 operations against 14 (1000 x 749: 50.6 us against 87, of which
 // the pipe needs 41).
-#include "yk_ff.cuh"
+#include "yk_cluster.cuh"
 #include "yk_kernels.h"
 
 namespace yk {
@@ -235,10 +235,16 @@ static cudaError_t launch_t(const void* in, void* out, const double* sigma, cons
                             double m0, double g, double r, cudaStream_t stream)
 {
     // bands of up to four rows (two rows more are read for each, most of them from
-    // L2: FP32, 2048 x 2048, four rows 51.4 us, eight 53.3, two 54.5), fewer where
-    // the lattice would give each of the 152 SMs less than four blocks
+    // L2: FP32, 2048 x 2048, in an early form four rows 51.4 us, eight 53.3, two 54.5), fewer
+    // where the lattice would give each SM less than four blocks
     const int gx = (Nx + kBlock - 1) / kBlock;
-    int band = (int)((int64_t)gx * Nt / (4 * 152));
+    const int n_sm = once_per_device([] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 1;
+    });
+    int band = (int)((int64_t)gx * Nt / (4 * n_sm));
     band = band < 1 ? 1 : band > 4 ? 4 : band;
     // g and the diagonal's constant as float-float, by the host (NaN for a g that FP32 holds
     // with fewer bits or not at all: the kernel takes FP64 then)
