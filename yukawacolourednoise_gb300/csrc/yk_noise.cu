@@ -36,7 +36,7 @@ __device__ __forceinline__ double2 c_mul(double2 a, double2 w)
 struct FftStage {
     const double2* x;
     double2* y;
-    int N, M, s, sj, sc, nseq;
+    int N, M, lm, s, ls, sj, sc, nseq;   // M = 2^lm (lm < 0: no power of two)
     bool twiddle, inverse;
     const double2* tw;
 
@@ -47,30 +47,45 @@ struct FftStage {
         if (inverse) w.y = -w.y;
         return w;
     }
-    // output k of a butterfly
+    // output k of a butterfly, as it is stored
+    __device__ __forceinline__ void put(int p, int q, int r, int k, int c, double2 v) const
+    {
+        y[(q + s * (r * p + k)) * sj + c * sc] = v;
+    }
     __device__ __forceinline__ void out(int p, int q, int r, int k, int c, double2 v) const
     {
-        if (twiddle && k > 0) v = c_mul(v, root(p * k * s));
-        y[(q + s * (r * p + k)) * sj + c * sc] = v;
+        put(p, q, r, k, c, twiddle && k > 0 ? c_mul(v, root(p * k * s)) : v);
     }
 };
 
-__device__ __forceinline__ void fft_even(const FftStage& f, int r)   // r = 4 or 2
+// r = 4 or 2: the first stages, so that s is a power of two, 2^ls.  A butterfly's loads go
+// before its arithmetic and its stores after it: a short transform is bound by their latency and
+// that of integer divisions, and the compiler moves no twiddle's load over a store that may alias it
+// (256 x 256, the noise in all: 43.0 us with each output's twiddle loaded at its store, 37.0 so).
+__device__ __forceinline__ void fft_even(const FftStage& f, int r)
 {
     for (int idx = threadIdx.x; idx < f.M * f.nseq; idx += blockDim.x) {
-        const int c = idx / f.M, b = idx - c * f.M, p = b / f.s, q = b - p * f.s;
+        const int c = f.lm >= 0 ? idx >> f.lm : idx / f.M, b = idx - c * f.M, p = b >> f.ls, q = b & (f.s - 1);
+        double2 w[4];
+        if (f.twiddle)
+#pragma unroll
+            for (int k = 1; k < 4; ++k)
+                if (k < r) w[k] = f.root(p * k * f.s);
         const double2 a0 = f.in(b, 0, c), a1 = f.in(b, 1, c);
         if (r == 4) {
             const double2 a2 = f.in(b, 2, c), a3 = f.in(b, 3, c);
             const double2 t0 = c_add(a0, a2), t1 = c_sub(a0, a2), t2 = c_add(a1, a3), d = c_sub(a1, a3);
             const double2 t3 = f.inverse ? make_double2(-d.y, d.x) : make_double2(d.y, -d.x);
-            f.out(p, q, 4, 0, c, c_add(t0, t2));
-            f.out(p, q, 4, 1, c, c_add(t1, t3));
-            f.out(p, q, 4, 2, c, c_sub(t0, t2));
-            f.out(p, q, 4, 3, c, c_sub(t1, t3));
+            double2 o[4] = {c_add(t0, t2), c_add(t1, t3), c_sub(t0, t2), c_sub(t1, t3)};
+            if (f.twiddle)
+#pragma unroll
+                for (int k = 1; k < 4; ++k) o[k] = c_mul(o[k], w[k]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) f.put(p, q, 4, k, c, o[k]);
         } else {
-            f.out(p, q, 2, 0, c, c_add(a0, a1));
-            f.out(p, q, 2, 1, c, c_sub(a0, a1));
+            const double2 o = c_sub(a0, a1);
+            f.put(p, q, 2, 0, c, c_add(a0, a1));
+            f.put(p, q, 2, 1, c, f.twiddle ? c_mul(o, w[1]) : o);
         }
     }
 }
@@ -104,11 +119,11 @@ __device__ __forceinline__ void fft_odd(const FftStage& f, int r)
 // holds the result.  tw[k] = exp(-2 pi i k / N), k < N.  Bound by the FP64 pipe:
 // a prime r costs about 4 r operations a point, so that a length with small
 // factors is far from a direct sum's 4 N (the noise of a 160 x 224 step in all:
-// 291 us by direct sums, 53 so).
+// 292 us by direct sums, 41 so).
 __device__ double2* smem_fft(double2* buf, double2* tmp, int N, int nseq, int sj, int sc,
                              const double2* __restrict__ tw, bool inverse)
 {
-    int n = N, s = 1, prime = 3;
+    int n = N, s = 1, ls = 0, prime = 3;
     while (n > 1) {
         int r;
         if (n % 4 == 0) {
@@ -119,13 +134,16 @@ __device__ double2* smem_fft(double2* buf, double2* tmp, int N, int nseq, int sj
             while (n % prime) prime = prime * prime > n ? n : prime + 2;
             r = prime;
         }
-        const FftStage f = {buf, tmp, N, N / r, s, sj, sc, nseq, n > r, inverse, tw};
-        if (r & 1)
-            fft_odd(f, r);
-        else
-            fft_even(f, r);
+        if (r & 1) {
+            fft_odd(FftStage{buf, tmp, N, N / r, 0, s, 0, sj, sc, nseq, n > r, inverse, tw}, r);
+            n /= r;
+        } else {
+            const int M = N >> (r >> 1), lm = (M & (M - 1)) == 0 ? __ffs(M) - 1 : -1;
+            fft_even(FftStage{buf, tmp, N, M, lm, s, ls, sj, sc, nseq, n > r, inverse, tw}, r);
+            n >>= r >> 1;
+            ls += r >> 1;
+        }
         __syncthreads();
-        n /= r;
         s *= r;
         double2* const q = buf;
         buf = tmp;
