@@ -5,15 +5,17 @@
 // rows, with rows t - 1, t, t + 1 in registers and row t + 2 on its way, so that
 // every site is read from memory about once; the x neighbours come from the next
 // lanes by warp shuffles (the lanes at a warp's and a row's ends load theirs).  The
+// columns of all bands are dealt out to the threads one after another, so that narrow lattices
+// leave no lanes idle (4096 x 2, FP64: 73.8 us with blocks of their own for each band, 7.6 so).  The
 // antiperiodic time signs and neighbour indices are computed instead of read from
 // IUP/IDN tables, and the output is written once (the reference zeroes `out`, adds
 // the diagonal and adds the hops in three grid-synced passes).  Complex (K = 2)
 // applies add the pion term g i gamma5 tau.pi when the chain carries pions.
 //
-// FP32 is bound by HBM (2048 x 2048: 43.9 us, 6.9 TB/s; its diagonal in float-float
+// FP32 is bound by HBM (2048 x 2048: 45.1 us, 6.7 TB/s; its diagonal in float-float
 // on the FP32 pipes), FP64 by its pipe, 1/64 of the FP32 rate: at r = 1 a time hop
 // keeps one spin entry and an x hop a combination u -+ d, so that a spin pair and
-// plane takes 8 operations against 14 (1000 x 749: 50.6 us against 87, of which
+// plane takes 8 operations against 14 (1000 x 749: 47.2 us against 87, of which
 // the pipe needs 41).
 #include "yk_cluster.cuh"
 #include "yk_kernels.h"
@@ -77,11 +79,19 @@ __device__ __forceinline__ XPart<R, K, R1> x_part(const Unit<R, K>& c, R s)   //
     return o;
 }
 
+// -c where `yes`.  In FP64 by the sign bits: lanes differ, and a negation that is selected
+// takes the FP64 pipe in all of them (1000 x 749: 58.6 us against 47.3; FP32 has it for nothing).
 template <typename R, int K>
-__device__ __forceinline__ void negate(Unit<R, K>& c)
+__device__ __forceinline__ void negate_if(Unit<R, K>& c, bool yes)
 {
+    const unsigned m = yes ? 0x80000000u : 0u;
 #pragma unroll
-    for (int k = 0; k < 2 * K; ++k) c.v[k] = -c.v[k];
+    for (int k = 0; k < 2 * K; ++k) {
+        if constexpr (sizeof(R) == 8)
+            c.v[k] = __hiloint2double((int)((unsigned)__double2hiint(c.v[k]) ^ m), __double2loint(c.v[k]));
+        else
+            c.v[k] = yes ? -c.v[k] : c.v[k];
+    }
 }
 
 }  // namespace
@@ -89,14 +99,16 @@ __device__ __forceinline__ void negate(Unit<R, K>& c)
 template <typename R, int K, bool DAG, bool R1>
 __global__ void __launch_bounds__(kBlock) dirac_kernel(const R* __restrict__ in, R* __restrict__ out,
                                                        const double* __restrict__ sigma, const double* __restrict__ pi,
-                                                       int Nt, int Nx, int gx, int band, double diag0, double g, double r,
-                                                       float4 ff)
+                                                       int Nt, int Nx, int columns, int band, double diag0, double g,
+                                                       double r, float4 ff)
 {
     using Un = Unit<R, K>;
     constexpr int F = 2;   // flavours
     const int V = Nt * Nx, lane = threadIdx.x & 31;
-    const int by = blockIdx.x / gx, at = (blockIdx.x - by * gx) * blockDim.x + threadIdx.x;
-    const int x = min(at, Nx - 1);   // threads past the row repeat its last site's work
+    const int at = blockIdx.x * kBlock + threadIdx.x;
+    if (at - lane >= columns) return;
+    const int col = min(at, columns - 1);   // the last warp's lanes past the last column repeat its work
+    const int by = col / Nx, x = col - by * Nx;
     // the x neighbours come from the lanes but at the ends
     const bool ld_up = lane == 31 || x == Nx - 1, ld_dn = lane == 0 || x == 0;
     const int x_up = x == Nx - 1 ? 0 : x + 1, x_dn = x == 0 ? Nx - 1 : x - 1;
@@ -115,11 +127,11 @@ __global__ void __launch_bounds__(kBlock) dirac_kernel(const R* __restrict__ in,
     };
     Part prev = load(t0 - 1, x), cur = load(t0, x), next = load(t0 + 1, x);
     double sg = sigma[t0 * Nx + x];
-    if (t0 == 0)
 #pragma unroll
-        for (int q = 0; q < F; ++q) negate(prev.u[q]);
-    for (int t = t0; t < t1; ++t) {
-        const int n = t * Nx + x;
+    for (int q = 0; q < F; ++q) negate_if(prev.u[q], t0 == 0);
+    // as many rows in every lane, for the shuffles: those past a shorter last band are not stored
+    for (int k = 0; k < band; ++k) {
+        const int t = t0 + k, n = min(t, Nt - 1) * Nx + x;
         Part ahead = next;
         double sg_ahead = sg;
         if (t + 1 < t1) {
@@ -127,9 +139,8 @@ __global__ void __launch_bounds__(kBlock) dirac_kernel(const R* __restrict__ in,
             sg_ahead = sigma[n + Nx];
         }
         XPart<R, K, R1> up[F], dn[F];
-        if (t + 1 == Nt)
 #pragma unroll
-            for (int q = 0; q < F; ++q) negate(next.u[q]);
+        for (int q = 0; q < F; ++q) negate_if(next.u[q], t + 1 == Nt);
         if constexpr (sizeof(R) == 4) {
 #pragma unroll
             for (int q = 0; q < F; ++q) {
@@ -220,7 +231,7 @@ __global__ void __launch_bounds__(kBlock) dirac_kernel(const R* __restrict__ in,
                 for (int q = 0; q < F; ++q)
                     unit_pions<R>(o.u[q], cur.u[q], cur.u[F - 1 - q], q, s1, s2, s3);
             }
-        if (at < Nx)
+        if (at < columns && t < t1)
 #pragma unroll
             for (int q = 0; q < F; ++q) st_unit<R, K>(out, (int64_t)n * F + q, o.u[q]);
         prev = cur;
@@ -237,22 +248,23 @@ static cudaError_t launch_t(const void* in, void* out, const double* sigma, cons
     // bands of up to four rows (two rows more are read for each, most of them from
     // L2: FP32, 2048 x 2048, in an early form four rows 51.4 us, eight 53.3, two 54.5), fewer
     // where the lattice would give each SM less than four blocks
-    const int gx = (Nx + kBlock - 1) / kBlock;
     const int n_sm = once_per_device([] {
         int dev = 0, n = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
         return n > 0 ? n : 1;
     });
-    int band = (int)((int64_t)gx * Nt / (4 * n_sm));
+    int band = (int)((int64_t)Nt * Nx / (4 * kBlock * n_sm));
     band = band < 1 ? 1 : band > 4 ? 4 : band;
+    if (band > Nt) band = Nt;   // (a lane past the last row wraps its loads once)
+    const int columns = (Nt + band - 1) / band * Nx;
     // g and the diagonal's constant as float-float, by the host (NaN for a g that FP32 holds
     // with fewer bits or not at all: the kernel takes FP64 then)
     const double diag0 = 2.0 * r + m0;
     const float gh = g == 0.0 || (fabs(g) > 0x1p-100 && fabs(g) < 0x1p100) ? (float)g : NAN, dh = (float)diag0;
     const float4 ff = make_float4(gh, (float)(g - gh), dh, (float)(diag0 - dh));
-    dirac_kernel<R, K, DAG, R1><<<gx * ((Nt + band - 1) / band), kBlock, 0, stream>>>(
-        (const R*)in, (R*)out, sigma, pi, Nt, Nx, gx, band, diag0, g, r, ff);
+    dirac_kernel<R, K, DAG, R1><<<(columns + kBlock - 1) / kBlock, kBlock, 0, stream>>>(
+        (const R*)in, (R*)out, sigma, pi, Nt, Nx, columns, band, diag0, g, r, ff);
     return cudaGetLastError();
 }
 
