@@ -556,6 +556,7 @@ struct FusedLayers {
 
 constexpr int kPmMaxConv = 16;              // 2L of pcg_m_kernel
 constexpr size_t kPmMaxSmem = 200 * 1024;   // its shared memory
+constexpr size_t kPmTwoSmem = 112 * 1024;   // with which two of its blocks share an SM
 __host__ __device__ inline size_t pm_smem(int R, int W, int H)
 {
     // the two activation buffers, r' and sigma of the tile, the fragments
@@ -913,7 +914,11 @@ LearnedNet* net_create(int Nt, int Nx, int layers, cudaError_t* err)
             int R = kTcMaxR, W = std::min(Nx, kTcMaxW);
             auto tiles = [&] { return ((Nt + R - 1) / R) * ((Nx + W - 1) / W); };
             while (tiles() < n_sm / 2 && (W > 16 || R > 2)) (W > 4 * R && W > 16 ? W : R) /= 2;
-            if (pm_smem(R, W, 2 * layers) <= kPmMaxSmem) {
+            // a layer's units and the waits between layers of one block leave an SM idle:
+            // from six layers on, whose halos leave room for one, only where every tile has an SM
+            // (us a step, 64 iterations, and one launch a phase: 512 x 512 five layers 5080
+            // and 6103, six 7974 and 6948; 256 x 256, 128 tiles, eight layers 3405 and 4691)
+            if (pm_smem(R, W, 2 * layers) <= (tiles() <= n_sm ? kPmMaxSmem : kPmTwoSmem)) {
                 n->pm_R = R;
                 n->pm_W = W;
                 n->pm_tiles = tiles();
