@@ -24,7 +24,7 @@ def test_time(ylib, cuda, monkeypatch, Nt, Nx, layers):
             ctx.set_field(sig)
             ctx.net_setup(layers=layers, seed=1)
             ctx.step_learned(6, True)   # the trials of the first solves
-            for _ in range(4):
+            for _ in range(10):
                 t = time.perf_counter()
                 ctx.step_learned(2, True)
                 ctx.synchronize()
